@@ -243,6 +243,15 @@ double optimize_layout(float* emb, int64_t n_vertices, int dim, const Graph& g, 
                        uint64_t seed, bool count_samples, float* kernel_ms, cudaStream_t s,
                        const DensityParams* dens = nullptr);
 
+// -------------------------------------------------------- sgd_small.cu
+// Graphs with n_vertices x dim up to this many floats take the deterministic
+// layout without densMAP: two copies of the embedding and one counter per
+// vertex fit one SM's shared memory.
+constexpr int64_t kSmallLayoutFloats = 16384;
+double optimize_layout_small(float* emb, int64_t n_vertices, int dim, const Graph& g,
+                             int64_t n_epochs, float a, float b, float lr, int64_t neg_rate,
+                             float repulsion, uint64_t seed, float* kernel_ms, cudaStream_t s);
+
 // local_radii_from_knn / embedding_radii_from_knn (lib.rs:5057-5108) and
 // density_start_epoch (lib.rs:5052-5055).
 void local_radii(const int32_t* idx, const float* dist, int64_t n, int k, float var_shift,
