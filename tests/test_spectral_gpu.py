@@ -59,3 +59,50 @@ def test_mixture_components_follow_oracle_layout(orc):
     # component anchors are deterministic (meta layout); within-component
     # coordinates agree up to the eigenvector sign per component
     np.testing.assert_allclose(g.mean(0), o.mean(0), atol=0.5)
+
+
+def hub_graph(n_blocks=5, seed=3):
+    """Blocks of random edges, loosely joined, with rows whose lengths lie at
+    the edges of the product's quads, chunks and row kinds."""
+    rng = np.random.default_rng(seed)
+    sizes = [230 + 30 * b for b in range(n_blocks)]
+    start = np.concatenate([[0], np.cumsum(sizes)])
+    n = int(start[-1])
+    w = np.zeros((n, n), np.float32)
+    for b, sz in enumerate(sizes):
+        i = start[b] + np.repeat(np.arange(sz), 12)
+        j = start[b] + rng.integers(0, sz, i.shape[0])
+        w[i, j] = rng.uniform(0.3, 1.0, i.shape[0])
+    for b, c in enumerate(range(1, n_blocks)):
+        i = start[b] + rng.integers(0, sizes[b], 80 + 60 * b)
+        j = start[c] + rng.integers(0, sizes[c], 80 + 60 * b)
+        w[i, j] = 0.5
+    w = np.maximum(w, w.T)
+    np.fill_diagonal(w, 0.0)
+    want = [95, 96, 97, 127, 128, 129, 255, 256, 257]
+    hubs = start[-2] + 3 + 7 * np.arange(len(want))
+    for row, length in zip(hubs, want):  # grown by edges to rows that are no hubs
+        free = [j for j in range(start[-2], n) if j not in hubs and j != row and w[row, j] == 0]
+        add = rng.choice(free, length - int((w[row] > 0).sum()), replace=False)
+        w[row, add] = w[add, row] = rng.uniform(0.3, 1.0, add.shape[0])
+    assert [int((w[r] > 0).sum()) for r in hubs] == want
+    return w
+
+
+@pytest.mark.parametrize("dim", [1, 2, 3, 4])
+def test_long_rows_give_the_dense_eigenvectors(dim):
+    w = hub_graph()
+    h, t = np.nonzero(w)
+    deg = w.astype(np.float64).sum(1)
+    a = w / np.sqrt(deg[:, None] * deg[None, :])
+    val, vec = np.linalg.eigh(a)
+    assert np.min(-np.diff(val[::-1][:dim + 2])) > 1e-3  # separated eigenvalues
+    x = np.zeros((w.shape[0], 16), np.float32)
+    g, used = gu.spectral_init(x, h.astype(np.int32), t.astype(np.int32), w[h, t], dim, 42)
+    assert used
+    ref = vec[:, ::-1][:, 1:dim + 1]
+    ref = ref * 10.0 / np.abs(ref).max()
+    ref = ref * np.sign((ref * g).sum(0))
+    # N(0, 1e-4) noise on every coordinate (6 sigma), FP32 products (6e-8)
+    # over eigenvalue gaps of 1e-3 at a scale of 10
+    assert np.abs(g - ref).max() < 6e-4 + 10 * 6e-8 / 1e-3 * 2

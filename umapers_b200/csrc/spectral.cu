@@ -48,6 +48,13 @@ constexpr double kOrthoEps = 1e-12;     // lib.rs:34
 constexpr float kInitMaxCoord = 10.0f;  // lib.rs:22
 constexpr float kInitNoise = 1e-4f;     // lib.rs:23
 constexpr int kMaxS = 32;               // s <= 32 -> n_components <= 4
+// Edges above which a row of a product takes a CTA: a row a short path walks
+// costs about 0.09 us per edge whatever the others do, so rows are long where
+// that would outlast a quarter of the whole product (10 ps per edge), but not
+// below 96 edges, where a CTA costs as much as the walk.  At 1M x 64 a fixed 96
+// made the products 99 ms a fit, the rule (671) 88.
+constexpr int32_t kLongRowMin = 96, kLongRowMax = 1024;
+constexpr int64_t kEdgesPerLongEdge = 36000;
 
 inline unsigned grid_for(int64_t n, int t = 256) {
     return static_cast<unsigned>(ceil_div(std::max<int64_t>(n, 1), t));
@@ -133,28 +140,40 @@ __global__ void pos_kernel(const int32_t* __restrict__ nodes, int64_t cnt, int32
     if (p < cnt) pos[nodes[p]] = static_cast<int32_t>(p);
 }
 
+// The CSR of the shifted operator in position order.  A row's edges start at
+// a multiple of four (rows are padded to whole quads), so four tails and four
+// weights arrive in one 16-byte load each.
 __global__ void prow_len_kernel(const int32_t* __restrict__ nodes, int64_t cnt,
-                                const int32_t* __restrict__ row_ptr, int32_t* __restrict__ len) {
+                                const int32_t* __restrict__ row_ptr, int32_t* __restrict__ len,
+                                int32_t* __restrict__ quads, int32_t long_row,
+                                int32_t* __restrict__ long_rows,
+                                int32_t* __restrict__ n_long) {
     const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (p < cnt) {
         const int32_t v = nodes[p];
-        len[p] = row_ptr[v + 1] - row_ptr[v];
+        const int32_t l = row_ptr[v + 1] - row_ptr[v];
+        len[p] = l;
+        quads[p] = (l + 3) / 4;
+        if (l > long_row) long_rows[atomicAdd(n_long, 1)] = static_cast<int32_t>(p);
     }
 }
 
-// CSR of the shifted operator in position order (tails mapped to positions).
 __global__ void pcsr_kernel(const int32_t* __restrict__ nodes, int64_t cnt,
                             const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ tails,
                             const float* __restrict__ nw, const int32_t* __restrict__ pos,
-                            const int32_t* __restrict__ prow_ptr, int32_t* __restrict__ ptails,
+                            const int32_t* __restrict__ qptr, int32_t* __restrict__ ptails,
                             float* __restrict__ pnw) {
     const int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (p >= cnt) return;
     const int32_t v = nodes[p];
-    int32_t o = prow_ptr[p];
+    int64_t o = static_cast<int64_t>(qptr[p]) * 4;
     for (int32_t e = row_ptr[v]; e < row_ptr[v + 1]; ++e, ++o) {
         ptails[o] = pos[tails[e]];
         pnw[o] = nw[e];
+    }
+    for (; o & 3; ++o) {  // padding: never used, but read
+        ptails[o] = static_cast<int32_t>(p);
+        pnw[o] = 0.0f;
     }
 }
 
@@ -177,37 +196,145 @@ __global__ void init_block_kernel(const int32_t* __restrict__ nodes, int64_t cnt
     }
 }
 
-// Y = X + A_hat X in position order.  SP / 4 lanes share a row, one float4
-// of it each, so every neighbour's row is gathered by one coalesced access;
-// each lane sums its components over the row's edges in edge order.
-template <int SP>
-__host__ __device__ constexpr int spmm_rows_per_warp() { return 32 / (SP / 4); }
+// Y = X + A_hat X in position order.  A row's sum adds its edges in edge
+// order, whatever path it takes.
+//
+// Short rows: SP / 4 lanes share a row, one float4 of it each, four edges at a
+// time, the next four tails and weights on the way.
+// Long rows: a CTA each, started first.  All threads gather the next
+// kLongChunk edges' rows while one warp, a lane per column, adds the previous
+// chunk from shared memory, so a hub costs about 7 cycles an edge instead of a
+// memory round trip for every four.
+constexpr int kSpmmThreads = 256;
+constexpr int kLongChunk = 128;
 
 template <int SP>
-__global__ void __launch_bounds__(256)
-    spmm_kernel(int64_t cnt, const int32_t* __restrict__ prow_ptr,
+constexpr int spmm_rows_per_block() { return kSpmmThreads / 32 * (32 / (SP / 4)); }
+
+template <int SP>
+__device__ __forceinline__ void spmm_long_row(int64_t t, const int32_t* __restrict__ qptr,
+                                              const int32_t* __restrict__ len,
+                                              const int32_t* __restrict__ ptails,
+                                              const float* __restrict__ pnw,
+                                              const float* __restrict__ X, float* __restrict__ Y) {
+    constexpr int V = SP / 4, GL = V <= 4 ? 4 : 8;  // lanes of a gathered row
+    constexpr int kGroups = kSpmmThreads / GL;
+    constexpr int kPer = kLongChunk / kGroups;  // edges a group gathers per chunk
+    __shared__ __align__(16) float tile[2][kLongChunk * SP];
+    __shared__ float wt[2][kLongChunk];
+    const int tid = threadIdx.x, grp = tid / GL, v = tid % GL;
+    const int32_t n = len[t];
+    const int64_t st = static_cast<int64_t>(qptr[t]) * 4;
+    float4 q[kPer];
+    float w[kPer];
+    int32_t id[kPer];
+    auto ids = [&](int32_t e0) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int32_t e = e0 + grp + k * kGroups;
+            id[k] = e < n ? __ldg(ptails + st + e) : -1;
+            w[k] = e < n ? __ldg(pnw + st + e) : 0.0f;
+        }
+    };
+    auto gather = [&] {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k)
+            if (v < V && id[k] >= 0)
+                q[k] = __ldg(reinterpret_cast<const float4*>(X + static_cast<int64_t>(id[k]) * SP) + v);
+    };
+    auto put = [&](int buf) {
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int e = grp + k * kGroups;
+            if (v < V && id[k] >= 0) reinterpret_cast<float4*>(tile[buf] + e * SP)[v] = q[k];
+            if (v == 0) wt[buf][e] = w[k];
+        }
+    };
+    float acc = tid < SP ? X[t * SP + tid] : 0.0f;
+    ids(0);
+    gather();
+    put(0);
+    for (int32_t e0 = 0; e0 < n; e0 += kLongChunk) {
+        const int buf = (e0 / kLongChunk) & 1;
+        const bool more = e0 + kLongChunk < n;
+        if (more) ids(e0 + kLongChunk);
+        __syncthreads();
+        if (more) gather();
+        if (tid < SP) {
+            const int32_t m = min(kLongChunk, n - e0);
+            int32_t e = 0;
+            for (; e + 8 <= m; e += 8) {
+                float x[8], a[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    x[k] = tile[buf][(e + k) * SP + tid];
+                    a[k] = wt[buf][e + k];
+                }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc = fmaf(a[k], x[k], acc);
+            }
+            for (; e < m; ++e) acc = fmaf(wt[buf][e], tile[buf][e * SP + tid], acc);
+        }
+        if (more) put(buf ^ 1);
+    }
+    if (tid < SP) Y[t * SP + tid] = acc;
+}
+
+template <int SP>
+__global__ void __launch_bounds__(kSpmmThreads, 4)
+    spmm_kernel(int64_t cnt, const int32_t* __restrict__ qptr, const int32_t* __restrict__ len,
                 const int32_t* __restrict__ ptails, const float* __restrict__ pnw,
+                const int32_t* __restrict__ long_rows, int n_long, int32_t long_row,
                 const float* __restrict__ X, float* __restrict__ Y) {
-    constexpr int V = SP / 4;
-    constexpr int RW = spmm_rows_per_warp<SP>();
+    if (static_cast<int>(blockIdx.x) < n_long) {
+        spmm_long_row<SP>(long_rows[blockIdx.x], qptr, len, ptails, pnw, X, Y);
+        return;
+    }
+    constexpr int V = SP / 4, RW = 32 / V;
     const int lane = threadIdx.x & 31;
     const int sub = lane / V, v = lane - sub * V;
-    const int64_t t =
-        ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * RW + sub;
+    const int64_t t = static_cast<int64_t>(blockIdx.x - n_long) * spmm_rows_per_block<SP>() +
+                      (threadIdx.x >> 5) * RW + sub;
     if (sub >= RW || t >= cnt) return;
-    float4 acc = reinterpret_cast<const float4*>(X + t * SP)[v];
-    const int32_t st = prow_ptr[t], en = prow_ptr[t + 1];
-#pragma unroll 4
-    for (int32_t e = st; e < en; ++e) {
-        const float wv = __ldg(pnw + e);
-        const float4 q =
-            __ldg(reinterpret_cast<const float4*>(X + static_cast<int64_t>(__ldg(ptails + e)) * SP) + v);
-        acc.x = fmaf(wv, q.x, acc.x);
-        acc.y = fmaf(wv, q.y, acc.y);
-        acc.z = fmaf(wv, q.z, acc.z);
-        acc.w = fmaf(wv, q.w, acc.w);
+    const int32_t n = len[t];
+    if (n > long_row) return;
+    const int32_t q0 = qptr[t];
+    const int4* id4 = reinterpret_cast<const int4*>(ptails) + q0;
+    const float4* w4 = reinterpret_cast<const float4*>(pnw) + q0;
+    const float4* x4 = reinterpret_cast<const float4*>(X);
+    float4 acc = x4[t * V + v];
+    auto add = [&](float w, const float4& q) {
+        acc.x = fmaf(w, q.x, acc.x);
+        acc.y = fmaf(w, q.y, acc.y);
+        acc.z = fmaf(w, q.z, acc.z);
+        acc.w = fmaf(w, q.w, acc.w);
+    };
+    auto row = [&](int32_t i) { return __ldg(x4 + static_cast<int64_t>(i) * V + v); };
+    int32_t e = 0;
+    if (n > 0) {
+        int4 id = __ldg(id4);
+        float4 w = __ldg(w4);
+#pragma unroll 1  // two quads at a time were 4% slower at 1M rows
+        for (; e + 4 <= n; e += 4) {
+            const float4 a = row(id.x), b = row(id.y), c = row(id.z), d = row(id.w);
+            const float4 wc = w;
+            if (e + 4 < n) {  // the next quad's tails and weights
+                id = __ldg(id4 + e / 4 + 1);
+                w = __ldg(w4 + e / 4 + 1);
+            }
+            add(wc.x, a);
+            add(wc.y, b);
+            add(wc.z, c);
+            add(wc.w, d);
+        }
+        if (e < n) {
+            const float4 a = row(id.x), b = row(id.y), c = row(id.z);  // padding reads its own row
+            add(w.x, a);
+            if (e + 1 < n) add(w.y, b);
+            if (e + 2 < n) add(w.z, c);
+        }
     }
-    reinterpret_cast<float4*>(Y + t * SP)[v] = acc;
+    reinterpret_cast<float4*>(Y)[t * V + v] = acc;
 }
 
 struct Chunk {
@@ -716,7 +843,8 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
         for (int k = 0; k < dim; ++k) slot_anchor[sl * dim + k] = multi ? anchors[c * dim + k] : 0.0f;
     }
     const int64_t cnt = static_cast<int64_t>(nodes_h.size());
-    DevBuf<int32_t> nodes(cnt, s), slots(cnt, s), pos(n, s), plen(cnt + 1, s), prow(cnt + 1, s);
+    DevBuf<int32_t> nodes(cnt, s), slots(cnt, s), pos(n, s), plen(cnt, s), quads(cnt + 1, s),
+        qptr(cnt + 1, s), long_rows(cnt, s), n_long(1, s);
     DevBuf<Chunk> dch(chunks.size(), s);
     DevBuf<uint64_t> dseed(n_slots, s), dnseed(n_slots, s);
     UMAPB_CUDA(cudaMemcpyAsync(nodes.get(), nodes_h.data(), cnt * 4, cudaMemcpyHostToDevice, s));
@@ -738,22 +866,29 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
     // position-ordered CSR
     pos_kernel<<<grid_for(cnt), 256, 0, s>>>(nodes.get(), cnt, pos.get());
     UMAPB_LAUNCH_CHECK();
-    prow_len_kernel<<<grid_for(cnt), 256, 0, s>>>(nodes.get(), cnt, g.row_ptr.get(), plen.get());
+    const int32_t long_row = static_cast<int32_t>(
+        std::max<int64_t>(kLongRowMin, std::min<int64_t>(kLongRowMax, m / kEdgesPerLongEdge)));
+    UMAPB_CUDA(cudaMemsetAsync(n_long.get(), 0, 4, s));
+    UMAPB_CUDA(cudaMemsetAsync(quads.get() + cnt, 0, 4, s));
+    prow_len_kernel<<<grid_for(cnt), 256, 0, s>>>(nodes.get(), cnt, g.row_ptr.get(), plen.get(),
+                                                  quads.get(), long_row, long_rows.get(),
+                                                  n_long.get());
     UMAPB_LAUNCH_CHECK();
-    UMAPB_CUDA(cudaMemsetAsync(plen.get() + cnt, 0, 4, s));
     {
         size_t tb = 0;
-        UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, plen.get(), prow.get(), cnt + 1, s));
+        UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, quads.get(), qptr.get(), cnt + 1, s));
         DevBuf<unsigned char> tmp(tb, s);
-        UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, plen.get(), prow.get(), cnt + 1, s));
+        UMAPB_CUDA(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, quads.get(), qptr.get(), cnt + 1, s));
     }
-    int32_t m_it = 0;
-    UMAPB_CUDA(cudaMemcpyAsync(&m_it, prow.get() + cnt, 4, cudaMemcpyDeviceToHost, s));
+    int32_t n_quads = 0, n_long_h = 0;
+    UMAPB_CUDA(cudaMemcpyAsync(&n_quads, qptr.get() + cnt, 4, cudaMemcpyDeviceToHost, s));
+    UMAPB_CUDA(cudaMemcpyAsync(&n_long_h, n_long.get(), 4, cudaMemcpyDeviceToHost, s));
     UMAPB_CUDA(cudaStreamSynchronize(s));
-    DevBuf<int32_t> ptails(std::max<int32_t>(m_it, 1), s);
-    DevBuf<float> pnw(std::max<int32_t>(m_it, 1), s);
+    const int64_t m_it = static_cast<int64_t>(n_quads) * 4;
+    DevBuf<int32_t> ptails(std::max<int64_t>(m_it, 4), s);
+    DevBuf<float> pnw(std::max<int64_t>(m_it, 4), s);
     pcsr_kernel<<<grid_for(cnt), 256, 0, s>>>(nodes.get(), cnt, g.row_ptr.get(), g.tails.get(),
-                                              nw.get(), pos.get(), prow.get(), ptails.get(), pnw.get());
+                                              nw.get(), pos.get(), qptr.get(), ptails.get(), pnw.get());
     UMAPB_LAUNCH_CHECK();
 
     DevBuf<float> Xb(cnt * SP, s), Yb(cnt * SP, s);
@@ -782,9 +917,11 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
         }
     };
     const unsigned gr_spmm = static_cast<unsigned>(
-        ceil_div(ceil_div(cnt, static_cast<int64_t>(spmm_rows_per_warp<SP>())) * 32, 256));
+        n_long_h + ceil_div(cnt, static_cast<int64_t>(spmm_rows_per_block<SP>())));
     auto spmm = [&](const float* x, float* y) {
-        spmm_kernel<SP><<<gr_spmm, 256, 0, s>>>(cnt, prow.get(), ptails.get(), pnw.get(), x, y);
+        spmm_kernel<SP><<<gr_spmm, kSpmmThreads, 0, s>>>(cnt, qptr.get(), plen.get(), ptails.get(),
+                                                         pnw.get(), long_rows.get(), n_long_h,
+                                                         long_row, x, y);
         UMAPB_LAUNCH_CHECK();
     };
     static_assert(kIters % kOrthoEvery == 0, "the last product must be orthonormalised");
