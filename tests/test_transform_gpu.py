@@ -53,3 +53,19 @@ def test_transform_out_buffer_empty_and_errors(fitted):
     bad[2, 1] = np.inf
     with pytest.raises(ValueError, match="non-finite value at row 2"):
         m.transform(bad)
+
+
+@pytest.mark.parametrize("k,rate", [(15, 5), (16, 12), (20, 5)])
+def test_transform_does_not_depend_on_the_lanes_per_query(k, rate):
+    # Small requests give a query 16, 8 or 4 lanes, larger ones one thread.
+    # Repeating a request's rows changes neither its largest weight nor its mean
+    # distance, and a row's random stream is keyed by its position, so the
+    # first copy's positions must come out the same bit for bit (rows of more
+    # than 16 edges and more than 8 negatives an edge take paths of their own).
+    fit, q = workloads.transform_mixture(n_fit=1500, n_query=9000, d=24, n_comp=6)
+    m = Umap(n_neighbors=k, n_epochs=20, negative_sample_rate=rate, random_seed=5)
+    m.fit(fit)
+    q[3] = fit[10]  # a fitted point
+    for n in (1, 31, 700, 4096, 4097, 8193):
+        whole = np.tile(q[:n], (16385 // n + 1, 1))
+        assert np.array_equal(m.transform(q[:n]), m.transform(whole)[:n])

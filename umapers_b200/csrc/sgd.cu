@@ -635,7 +635,9 @@ __device__ __forceinline__ void stage_query_2d(const TransformArgs& p, int32_t s
 // first collects the query's due edges in a bit mask, then serves them in
 // edge order: the lanes of a warp step through their own due edges together,
 // so a warp runs as many edge updates as its busiest query has due, not as
-// many as all 32 queries have together.
+// many as all 32 queries have together.  Negatives are applied from fixed
+// registers, with selects instead of branches around the update (1M queries:
+// 12.2 -> 10.0 ms).
 __device__ __forceinline__ void transform_schedule_2d_staged(const TransformArgs& p, int32_t st,
                                                              int cnt, uint64_t qseed,
                                                              TransformStage& sm, int tid,
@@ -690,30 +692,25 @@ __device__ __forceinline__ void transform_schedule_2d_staged(const TransformArgs
             }
             sm.next[j][tid] = __fadd_rn(nx, eps);
             if (!neg_ok) continue;
-            for (uint32_t s = 0; s < n_neg; ++s) {
-                float2 o;
-                if (s < static_cast<uint32_t>(kNegPrefetch)) {
-                    o = ng[0];
-#pragma unroll
-                    for (int t = 1; t < kNegPrefetch; ++t)
-                        if (s == static_cast<uint32_t>(t)) o = ng[t];
-                } else {
-                    const uint64_t word = rng_word(qseed, static_cast<uint64_t>(e - st),
-                                                   (static_cast<uint64_t>(epoch) << 32) | s);
-                    o = base[rng_below(word, p.n_base)];
-                }
+            auto repel = [&](const float2 o) {
                 const float dx = __fsub_rn(cx, o.x), dy = __fsub_rn(cy, o.y);
                 const float dd = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-                float g2 = 0.0f;
-                if (dd > 0.0f) {
-                    const float pb = pow_pos(dd, p.b);
-                    g2 = __fdiv_rn(rep, __fmul_rn(__fadd_rn(0.001f, dd),
-                                                  __fadd_rn(__fmul_rn(p.a, pb), 1.0f)));
-                }
-                if (g2 > 0.0f) {
-                    cx = __fadd_rn(cx, __fmul_rn(clip4(__fmul_rn(g2, dx)), alpha));
-                    cy = __fadd_rn(cy, __fmul_rn(clip4(__fmul_rn(g2, __fsub_rn(cy, o.y))), alpha));
-                }
+                const float pb = pow_pos(dd, p.b);
+                const float g2 = __fdiv_rn(
+                    rep, __fmul_rn(__fadd_rn(0.001f, dd), __fadd_rn(__fmul_rn(p.a, pb), 1.0f)));
+                const bool moves = dd > 0.0f && g2 > 0.0f;
+                const float nx = __fadd_rn(cx, __fmul_rn(clip4(__fmul_rn(g2, dx)), alpha));
+                const float ny = __fadd_rn(cy, __fmul_rn(clip4(__fmul_rn(g2, dy)), alpha));
+                cx = moves ? nx : cx;
+                cy = moves ? ny : cy;
+            };
+#pragma unroll
+            for (int s = 0; s < kNegPrefetch; ++s)
+                if (static_cast<uint32_t>(s) < n_neg) repel(ng[s]);
+            for (uint32_t s = kNegPrefetch; s < n_neg; ++s) {
+                const uint64_t word = rng_word(qseed, static_cast<uint64_t>(e - st),
+                                               (static_cast<uint64_t>(epoch) << 32) | s);
+                repel(base[rng_below(word, p.n_base)]);
             }
             sm.next_neg[j][tid] = __fadd_rn(nn, __fmul_rn(static_cast<float>(n_neg), eneg));
         }
@@ -722,24 +719,10 @@ __device__ __forceinline__ void transform_schedule_2d_staged(const TransformArgs
     cur[1] = cy;
 }
 
-__global__ void __launch_bounds__(kTransformThreads) transform_kernel(TransformArgs p) {
-    __shared__ TransformStage sm;
-    const int tid = threadIdx.x;
-    const int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid;
-    if (q >= p.nq) return;
+// init_graph_transform (lib.rs:4793-4836): the weighted mean of the query's
+// neighbours, or the first one of weight 1.
+__device__ void init_query(const TransformArgs& p, int32_t st, int32_t en, float* cur) {
     const int dim = p.dim;
-    const int32_t st = p.row_ptr[q], en = p.row_ptr[q + 1];
-    if (dim == 2 && en - st <= kStageEdges) {
-        float c2[2];
-        stage_query_2d(p, st, en - st, sm, tid, c2);
-        const uint64_t qseed = query_seed(p, q);
-        transform_schedule_2d_staged(p, st, en - st, qseed, sm, tid, c2);
-        p.out[q * 2] = c2[0];
-        p.out[q * 2 + 1] = c2[1];
-        return;
-    }
-    float cur[kMaxDim];
-    // init_graph_transform (lib.rs:4793-4836)
     if (st == en) {
         for (int c = 0; c < dim; ++c) cur[c] = NAN;
     } else {
@@ -766,6 +749,26 @@ __global__ void __launch_bounds__(kTransformThreads) transform_kernel(TransformA
             }
         }
     }
+}
+
+__global__ void __launch_bounds__(kTransformThreads) transform_kernel(TransformArgs p) {
+    __shared__ TransformStage sm;
+    const int tid = threadIdx.x;
+    const int64_t q = static_cast<int64_t>(blockIdx.x) * blockDim.x + tid;
+    if (q >= p.nq) return;
+    const int dim = p.dim;
+    const int32_t st = p.row_ptr[q], en = p.row_ptr[q + 1];
+    if (dim == 2 && en - st <= kStageEdges) {
+        float c2[2];
+        stage_query_2d(p, st, en - st, sm, tid, c2);
+        const uint64_t qseed = query_seed(p, q);
+        transform_schedule_2d_staged(p, st, en - st, qseed, sm, tid, c2);
+        p.out[q * 2] = c2[0];
+        p.out[q * 2 + 1] = c2[1];
+        return;
+    }
+    float cur[kMaxDim];
+    init_query(p, st, en, cur);
     // optimize_layout_transform (lib.rs:5444-5544)
     const uint64_t qseed = query_seed(p, q);
     if (dim == 2) {
@@ -826,6 +829,174 @@ __global__ void __launch_bounds__(kTransformThreads) transform_kernel(TransformA
         }
     }
     for (int c = 0; c < dim; ++c) p.out[q * dim + c] = cur[c];
+}
+
+// The same schedule with G lanes to a query (G divides kStageEdges).  Which
+// edges are due, their negative counts and the negatives do not depend on the
+// moving point, so each lane keeps the schedule of its own kStageEdges / G
+// edges in registers and, while the group works through one epoch's samples,
+// copies the next epoch's negatives into shared memory.  What is left on the
+// chain is the update itself (about 230 cycles a sample).
+constexpr int64_t kLanes16Queries = 4096, kLanes8Queries = 8192, kLanes4Queries = 16384;
+
+struct GroupStage {
+    float2 tail[kStageEdges];
+    float2 neg[2][kStageEdges][kNegPrefetch];
+    uint32_t n_neg[2][kStageEdges];
+    float w[kStageEdges];
+};
+
+template <int G>
+__global__ void __launch_bounds__(kTransformThreads) transform_group_kernel(TransformArgs p) {
+    constexpr int kPer = kStageEdges / G;
+    extern __shared__ __align__(16) uint8_t gsm[];
+    const int lane = threadIdx.x & 31, gl = lane % G, shift = lane - gl;
+    GroupStage& sm = reinterpret_cast<GroupStage*>(gsm)[threadIdx.x / G];
+    const int64_t q =
+        static_cast<int64_t>(blockIdx.x) * (kTransformThreads / G) + threadIdx.x / G;
+    const int32_t st = q < p.nq ? p.row_ptr[q] : 0, en = q < p.nq ? p.row_ptr[q + 1] : 0;
+    const bool wide = en - st > kStageEdges;  // the group's first lane takes the general loop
+    const int cnt = wide ? 0 : en - st;
+    const uint64_t qseed = q < p.nq ? query_seed(p, q) : 0;
+    const float2* base = reinterpret_cast<const float2*>(p.base);
+    float next[kPer], nneg[kPer], eps[kPer], eneg[kPer];
+    uint64_t stream[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+        const int j = k * G + gl;
+        if (j < cnt) {
+            sm.tail[j] = base[p.tails[st + j]];
+            sm.w[j] = p.weights[st + j];
+            eps[k] = p.eps[st + j];
+            next[k] = p.next[st + j];
+            nneg[k] = p.next_neg[st + j];
+            eneg[k] = __fdiv_rn(eps[k], p.neg_rate_f);
+        }
+        stream[k] = mix64(qseed ^ mix64(static_cast<uint64_t>(j)));
+    }
+    __syncwarp();
+    // init_graph_transform (lib.rs:4793-4836), on every lane of the group
+    float cx = NAN, cy = NAN;
+    if (cnt > 0) {
+        int copy_j = -1;
+        float sum = 0.0f;
+        for (int j = 0; j < cnt; ++j) {
+            if (copy_j < 0 && fabsf(__fsub_rn(sm.w[j], 1.0f)) < FLT_EPSILON) copy_j = j;
+            sum = __fadd_rn(sum, sm.w[j]);
+        }
+        if (copy_j >= 0) {
+            cx = sm.tail[copy_j].x;
+            cy = sm.tail[copy_j].y;
+        } else if (sum > 0.0f) {
+            cx = cy = 0.0f;
+            for (int j = 0; j < cnt; ++j) {
+                const float wj = __fdiv_rn(sm.w[j], sum);
+                cx = __fadd_rn(cx, __fmul_rn(wj, sm.tail[j].x));
+                cy = __fadd_rn(cy, __fmul_rn(wj, sm.tail[j].y));
+            }
+        }
+    }
+    // The due edges of `epoch` as a mask; starts the copies of their negatives.
+    auto plan = [&](int64_t epoch) {
+        uint32_t due = 0;
+        const float ef = static_cast<float>(epoch);
+        const int buf = static_cast<int>(epoch & 1);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int j = k * G + gl;
+            const bool mine = j < cnt && !(next[k] > ef);
+            if (mine) {
+                const bool neg_ok = isfinite(eneg[k]) && eneg[k] > 0.0f;
+                const uint32_t n =
+                    neg_ok ? floor_count(__fdiv_rn(__fsub_rn(ef, nneg[k]), eneg[k])) : 0u;
+                next[k] = __fadd_rn(next[k], eps[k]);
+                if (neg_ok) nneg[k] = __fadd_rn(nneg[k], __fmul_rn(static_cast<float>(n), eneg[k]));
+                sm.n_neg[buf][j] = n;
+#pragma unroll
+                for (int s = 0; s < kNegPrefetch; ++s)
+                    if (static_cast<uint32_t>(s) < n) {
+                        const uint64_t word =
+                            mix64(stream[k] ^ ((static_cast<uint64_t>(epoch) << 32) | s));
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                                         static_cast<uint32_t>(
+                                             __cvta_generic_to_shared(&sm.neg[buf][j][s]))),
+                                     "l"(base + rng_below(word, p.n_base))
+                                     : "memory");
+                    }
+            }
+            due |= ((__ballot_sync(0xffffffffu, mine) >> shift) & ((1u << G) - 1u)) << (k * G);
+        }
+        return due;
+    };
+    const float att = __fmul_rn(__fmul_rn(-2.0f, p.a), p.b);
+    const float rep = __fmul_rn(__fmul_rn(2.0f, p.rep), p.b);
+    bool alive = true;  // false once the point stopped being finite: nothing moves it then
+    uint32_t due = p.n_epochs > 0 ? plan(0) : 0u;
+    for (int64_t epoch = 0; epoch < p.n_epochs; ++epoch) {
+        const int buf = static_cast<int>(epoch & 1);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        uint32_t todo = due;
+        if (epoch + 1 < p.n_epochs) due = plan(epoch + 1);
+        const float alpha = __fmul_rn(
+            p.lr, __fsub_rn(1.0f, __fdiv_rn(static_cast<float>(epoch),
+                                            static_cast<float>(p.n_epochs))));
+        while (todo && alive) {
+            const int j = __ffs(todo) - 1;
+            todo &= todo - 1;
+            if (!(isfinite(cx) && isfinite(cy))) {
+                alive = false;
+                break;
+            }
+            const uint32_t n_neg = sm.n_neg[buf][j];
+            const float2 ot = sm.tail[j];
+            float2 o = sm.neg[buf][j][0];
+            {
+                const float dx = __fsub_rn(cx, ot.x), dy = __fsub_rn(cy, ot.y);
+                const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+                float gc = 0.0f;
+                if (d2 > 0.0f) {
+                    const float l2 = log2f(d2);
+                    const float pb = exp2f(__fmul_rn(p.b, l2));
+                    gc = __fdiv_rn(__fmul_rn(att, exp2f(__fmul_rn(p.b - 1.0f, l2))),
+                                   __fadd_rn(__fmul_rn(p.a, pb), 1.0f));
+                }
+                cx = __fadd_rn(cx, __fmul_rn(clip4(__fmul_rn(gc, dx)), alpha));
+                cy = __fadd_rn(cy, __fmul_rn(clip4(__fmul_rn(gc, dy)), alpha));
+            }
+            for (uint32_t s = 0; s < n_neg; ++s) {
+                float2 on = make_float2(0.0f, 0.0f);  // the next one, on the way meanwhile
+                if (s + 1 < static_cast<uint32_t>(kNegPrefetch)) {
+                    on = sm.neg[buf][j][s + 1];
+                } else if (s + 1 < n_neg) {
+                    const uint64_t word =
+                        rng_word(qseed, static_cast<uint64_t>(j),
+                                 (static_cast<uint64_t>(epoch) << 32) | (s + 1));
+                    on = base[rng_below(word, p.n_base)];
+                }
+                const float dx = __fsub_rn(cx, o.x), dy = __fsub_rn(cy, o.y);
+                const float dd = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
+                const float pb = pow_pos(dd, p.b);
+                const float g2 = __fdiv_rn(
+                    rep, __fmul_rn(__fadd_rn(0.001f, dd), __fadd_rn(__fmul_rn(p.a, pb), 1.0f)));
+                const bool moves = dd > 0.0f && g2 > 0.0f;
+                const float nx = __fadd_rn(cx, __fmul_rn(clip4(__fmul_rn(g2, dx)), alpha));
+                const float ny = __fadd_rn(cy, __fmul_rn(clip4(__fmul_rn(g2, dy)), alpha));
+                cx = moves ? nx : cx;
+                cy = moves ? ny : cy;
+                o = on;
+            }
+        }
+        __syncwarp();
+    }
+    if (q < p.nq && gl == 0) {
+        float c2[2] = {cx, cy};
+        if (wide) {
+            init_query(p, st, en, c2);
+            transform_schedule_2d(p, q, st, en, qseed, c2);
+        }
+        reinterpret_cast<float2*>(p.out)[q] = make_float2(c2[0], c2[1]);
+    }
 }
 
 // ------------------------------------------------------ inverse transform --
@@ -1275,8 +1446,29 @@ void transform_layout(float* out, int64_t nq, int dim, const float* base, int64_
     p.seed = seed;
     p.qid = qid;
     p.qid_offset = qid_offset;
-    transform_kernel<<<static_cast<unsigned>(ceil_div(nq, static_cast<int64_t>(kTransformThreads))),
-                       kTransformThreads, 0, s>>>(p);
+    auto group = [&](auto kernel, int lanes, size_t stage) {
+        const int64_t per_block = kTransformThreads / lanes;
+        const int smem = static_cast<int>(per_block * stage);
+        UMAPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        kernel<<<static_cast<unsigned>(ceil_div(nq, per_block)), kTransformThreads, smem, s>>>(p);
+    };
+    // A small request leaves SMs idle at one thread a query, and its time is one
+    // query's chain: the more lanes help, the shorter it is, as long as the
+    // schedulers keep a few warps each.  100 epochs on a 4,000-row fit, ms at
+    // 1 / 3,000 / 6,000 / 10,000 queries: one thread 1.75 / 2.64 / 2.54 / 2.55, 4
+    // lanes 1.29 / 1.80 / 1.88 / 2.13, 8 lanes 1.18 / 1.65 / 1.79 / 2.49, 16 lanes
+    // 1.11 / 1.54 / 2.51 / 3.56; 30 epochs at 35,000 queries: one thread 0.72,
+    // 4 lanes 1.48.
+    if (dim == 2 && nq <= kLanes16Queries)
+        group(transform_group_kernel<16>, 16, sizeof(GroupStage));
+    else if (dim == 2 && nq <= kLanes8Queries)
+        group(transform_group_kernel<8>, 8, sizeof(GroupStage));
+    else if (dim == 2 && nq <= kLanes4Queries)
+        group(transform_group_kernel<4>, 4, sizeof(GroupStage));
+    else
+        transform_kernel<<<static_cast<unsigned>(
+                               ceil_div(nq, static_cast<int64_t>(kTransformThreads))),
+                           kTransformThreads, 0, s>>>(p);
     UMAPB_LAUNCH_CHECK();
 }
 
