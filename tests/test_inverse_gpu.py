@@ -74,3 +74,25 @@ def test_inverse_transform_contracts():
     ms = Umap(n_neighbors=10, n_epochs=30).fit(sp.csr_matrix(x))
     with pytest.raises(ValueError, match="not supported for sparse-trained models"):
         ms.inverse_transform(np.zeros((2, 2), np.float32))
+
+
+@pytest.mark.parametrize("d,rate", [(1, 5), (24, 5), (32, 40), (33, 5), (64, 5), (65, 12), (128, 5),
+                                    (129, 5), (256, 5)])
+def test_inverse_in_registers_equals_the_general_path(orc, d, rate):
+    # Rows of up to 256 columns are kept in registers.  Zero columns change no
+    # distance, so the same rows padded to 288 columns, which take the general
+    # path, give the same positions bit for bit.  Both models are fitted from
+    # the same neighbour lists and random positions.
+    rng = np.random.default_rng(d)
+    x = rng.normal(0, 1.5, (300, d)).astype(np.float32)
+    wide = np.zeros((300, 288), np.float32)
+    wide[:, :d] = x
+    idx, dist = orc.exact_knn(x, 10)
+    kw = dict(n_neighbors=10, n_epochs=60, init="random", negative_sample_rate=rate)
+    a, b = Umap(**kw), Umap(**kw)
+    ea = a.fit_transform_with_knn(x, idx, dist)
+    assert np.array_equal(ea, b.fit_transform_with_knn(wide, idx, dist))
+    z = (ea[rng.integers(0, 300, 77)] + rng.normal(0, 0.2, (77, 2))).astype(np.float32)
+    z[5] = ea[9]
+    ra, rb = a.inverse_transform(z), b.inverse_transform(z)
+    assert np.array_equal(ra, rb[:, :d]) and not rb[:, d:].any()
