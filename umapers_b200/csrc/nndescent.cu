@@ -52,6 +52,18 @@ __device__ inline void warp_sort_u64(uint64_t* a, int cap) {
     }
 }
 
+// The distance of rows i and j from their squared distance or dot product.
+__device__ __forceinline__ float dense_distance(float sum, const float* __restrict__ norms,
+                                                int64_t i, int64_t j, bool cosine) {
+    if (!cosine) return __fsqrt_rn(sum);
+    const float xn = norms[i], yn = norms[j];
+    if (xn == 0.0f && yn == 0.0f) return 0.0f;
+    if (xn == 0.0f || yn == 0.0f) return 1.0f;
+    float cs = __fdiv_rn(sum, __fmul_rn(xn, yn));
+    cs = fminf(fmaxf(cs, -1.0f), 1.0f);
+    return __fsub_rn(1.0f, cs);
+}
+
 // Distance of query row i (in shared memory `qs`) to the candidates in
 // keys[0, m) (row indices), written back in place as (distance, index) keys.
 // Every lane of the warp calls it with the same m.
@@ -73,22 +85,7 @@ __device__ inline void eval_candidates(const float* __restrict__ X, const float*
                     sum = __fadd_rn(sum, __fmul_rn(df, df));
                 }
             }
-            float dist;
-            if (!cosine) {
-                dist = __fsqrt_rn(sum);
-            } else {
-                const float xn = norms[i], yn = norms[j];
-                if (xn == 0.0f && yn == 0.0f) {
-                    dist = 0.0f;
-                } else if (xn == 0.0f || yn == 0.0f) {
-                    dist = 1.0f;
-                } else {
-                    float cs = __fdiv_rn(sum, __fmul_rn(xn, yn));
-                    cs = fminf(fmaxf(cs, -1.0f), 1.0f);
-                    dist = __fsub_rn(1.0f, cs);
-                }
-            }
-            keys[c] = knn_key(dist, static_cast<uint32_t>(j));
+            keys[c] = knn_key(dense_distance(sum, norms, i, j, cosine), static_cast<uint32_t>(j));
         }
         return;
     }
@@ -121,22 +118,7 @@ __device__ inline void eval_candidates(const float* __restrict__ X, const float*
                     sum = __fadd_rn(sum, __fmul_rn(df, df));
                 }
             }
-            float dist;
-            if (!cosine) {
-                dist = __fsqrt_rn(sum);
-            } else {
-                const float xn = norms[i], yn = norms[j];
-                if (xn == 0.0f && yn == 0.0f) {
-                    dist = 0.0f;
-                } else if (xn == 0.0f || yn == 0.0f) {
-                    dist = 1.0f;
-                } else {
-                    float cs = __fdiv_rn(sum, __fmul_rn(xn, yn));
-                    cs = fminf(fmaxf(cs, -1.0f), 1.0f);
-                    dist = __fsub_rn(1.0f, cs);
-                }
-            }
-            keys[c] = knn_key(dist, static_cast<uint32_t>(j));
+            keys[c] = knn_key(dense_distance(sum, norms, i, j, cosine), static_cast<uint32_t>(j));
         }
     }
 }
@@ -152,54 +134,52 @@ struct NdCsr {
     int max_nnz;
 };
 
-// Distance of CSR row i (its columns and values in shared memory) to the
-// candidates in keys[0, m), one lane per candidate: the sparse dot is a
-// merge of the two sorted column lists, products of shared columns added in
-// ascending column order from +0.0 (sparse_dot, sparse.rs:220-239), and the
-// distance comes from it and the norms as in the exact sparse kNN
-// (sparse.rs:605-626); a row's distance to itself is 0 (sparse.rs:614-617).
+// Distance of CSR row i (its columns and values in shared memory) to row j:
+// the sparse dot is a merge of the two sorted column lists, products of shared
+// columns added in ascending column order from +0.0 (sparse_dot,
+// sparse.rs:220-239), and the distance comes from it and the norms as in the
+// exact sparse kNN (sparse.rs:605-626); a row's distance to itself is 0
+// (sparse.rs:614-617).
+__device__ inline float csr_distance(const NdCsr& x, int64_t i, int64_t j, int metric,
+                                     const int32_t* qc, const float* qv, int qn) {
+    if (j == i) return 0.0f;
+    float dot = 0.0f;
+    int a = 0;
+    int64_t b = x.ptr[j];
+    const int64_t be = x.ptr[j + 1];
+    while (a < qn && b < be) {
+        const int32_t ca = qc[a], cb = x.idx[b];
+        if (ca == cb) {
+            dot = __fadd_rn(dot, __fmul_rn(qv[a], x.val[b]));
+            ++a;
+            ++b;
+        } else if (ca < cb) {
+            ++a;
+        } else {
+            ++b;
+        }
+    }
+    if (metric == UMAPB_METRIC_COSINE) {
+        const float q_l2 = x.l2[i], r_l2 = x.l2[j];
+        if (q_l2 == 0.0f && r_l2 == 0.0f) return 0.0f;
+        if (q_l2 == 0.0f || r_l2 == 0.0f) return 1.0f;
+        float cs = __fdiv_rn(dot, __fmul_rn(q_l2, r_l2));
+        cs = fminf(fmaxf(cs, -1.0f), 1.0f);
+        return __fsub_rn(1.0f, cs);
+    }
+    float t = __fsub_rn(__fadd_rn(x.sq[i], x.sq[j]), __fmul_rn(2.0f, dot));
+    if (!(t > 0.0f)) t = 0.0f;
+    return __fsqrt_rn(t);
+}
+
+// The distances of CSR row i to the candidates in keys[0, m), one lane per
+// candidate, written back as (distance, index) keys.
 __device__ inline void eval_candidates_csr(const NdCsr& x, int64_t i, int metric, const int32_t* qc,
                                            const float* qv, int qn, uint64_t* keys, int m) {
     const int lane = threadIdx.x & 31;
-    const float q_sq = x.sq[i], q_l2 = x.l2[i];
     for (int c = lane; c < m; c += 32) {
         const int64_t j = static_cast<int64_t>(keys[c]);
-        float dist = 0.0f;
-        if (j != i) {
-            float dot = 0.0f;
-            int a = 0;
-            int64_t b = x.ptr[j];
-            const int64_t be = x.ptr[j + 1];
-            while (a < qn && b < be) {
-                const int32_t ca = qc[a], cb = x.idx[b];
-                if (ca == cb) {
-                    dot = __fadd_rn(dot, __fmul_rn(qv[a], x.val[b]));
-                    ++a;
-                    ++b;
-                } else if (ca < cb) {
-                    ++a;
-                } else {
-                    ++b;
-                }
-            }
-            if (metric == UMAPB_METRIC_COSINE) {
-                const float r_l2 = x.l2[j];
-                if (q_l2 == 0.0f && r_l2 == 0.0f) {
-                    dist = 0.0f;
-                } else if (q_l2 == 0.0f || r_l2 == 0.0f) {
-                    dist = 1.0f;
-                } else {
-                    float cs = __fdiv_rn(dot, __fmul_rn(q_l2, r_l2));
-                    cs = fminf(fmaxf(cs, -1.0f), 1.0f);
-                    dist = __fsub_rn(1.0f, cs);
-                }
-            } else {
-                float t = __fsub_rn(__fadd_rn(q_sq, x.sq[j]), __fmul_rn(2.0f, dot));
-                if (!(t > 0.0f)) t = 0.0f;
-                dist = __fsqrt_rn(t);
-            }
-        }
-        keys[c] = knn_key(dist, static_cast<uint32_t>(j));
+        keys[c] = knn_key(csr_distance(x, i, j, metric, qc, qv, qn), static_cast<uint32_t>(j));
     }
 }
 
@@ -223,6 +203,7 @@ struct NdArgs {
     unsigned long long* evaluated;  // kEvalSlots counters of candidates evaluated
     NdCsr csr;                       // sparse rows (the SP kernels)
     int metric;
+    bool quads;                      // dense rows are whole, aligned 16-byte quads
 };
 
 constexpr int kEvalSlots = 64;  // spread the per-warp counts over 64 addresses
@@ -378,6 +359,330 @@ __global__ void __launch_bounds__(kWarps * 32) nd_iter_kernel(NdArgs p, uint64_t
     if (__any_sync(0xffffffffu, diff) && lane == 0) *p.changed = 1;
 }
 
+// ------------------------------------------------ candidates in registers --
+// The iteration for k <= 31 (cap <= 1,024).  A warp's candidate indices live
+// in registers, NPL = cap / 32 consecutive ones a lane, through the sort and
+// the removal of duplicates; the random cut is worked out without running
+// its swaps one after another (a lane drew and swapped 201 times on its own);
+// distances load 16 bytes at a time; and the k best come from a 32-entry list
+// instead of a second sort.  Bound by the gathers of candidate rows:
+// 100,003 x 100 rows, k = 15, 50 candidates, 14 iterations (2.5e8 candidates of
+// 400 bytes) 38.6 -> 18.6 ms, 5.4 TB/s; 200,000 x 64, 10 iterations 42.8 -> 16.0;
+// 8,000 x 100, k = 30 7.6 -> 2.1; 20,000 CSR rows 5.2 -> 2.1.
+
+// Ascending bitonic sort of 32 * NPL values, element NPL * lane + r in v[r].
+template <int NPL>
+__device__ __forceinline__ void reg_sort_u32(uint32_t (&v)[NPL]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * NPL; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= NPL) {
+                const int ls = stride / NPL;
+                const bool up = size >= 32 * NPL || ((lane & (size / NPL)) == 0);
+                const bool keep_min = up == ((lane & ls) == 0);
+#pragma unroll
+                for (int r = 0; r < NPL; ++r) {
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], ls);
+                    v[r] = keep_min ? min(v[r], o) : max(v[r], o);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < NPL; ++r) {
+                    if ((r & stride) == 0) {
+                        const bool up = size < NPL ? (r & size) == 0
+                                                   : size >= 32 * NPL || (lane & (size / NPL)) == 0;
+                        const uint32_t a = v[r], b = v[r + stride];
+                        v[r] = up ? min(a, b) : max(a, b);
+                        v[r + stride] = up ? max(a, b) : min(a, b);
+                    }
+                }
+            }
+        }
+    }
+}
+
+// Keys above which a chunk is merged into the list of best keys in one
+// bitonic pass instead of one by one.
+constexpr int kInsertMost = 5;
+
+// The 32 smallest of the sorted list `best` and the 32 keys of `chunk` (any
+// order), sorted across the lanes.
+__device__ __forceinline__ uint64_t merge_best(uint64_t best, uint64_t chunk) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            const uint64_t o = __shfl_xor_sync(0xffffffffu, chunk, stride);
+            const bool keep_min = ((lane & size) == 0) == ((lane & stride) == 0);
+            chunk = keep_min ? (chunk < o ? chunk : o) : (chunk < o ? o : chunk);
+        }
+    }
+    const uint64_t rev = __shfl_sync(0xffffffffu, chunk, 31 - lane);
+    uint64_t x = best < rev ? best : rev;
+#pragma unroll
+    for (int st = 16; st > 0; st >>= 1) {
+        const uint64_t o = __shfl_xor_sync(0xffffffffu, x, st);
+        x = (lane & st) ? (x > o ? x : o) : (x < o ? x : o);
+    }
+    return x;
+}
+
+// The distances for rows that are not whole 16-byte quads: eval_candidates
+// on index and distance arrays.
+__device__ inline void eval_scalar(const float* __restrict__ X, const float* __restrict__ norms,
+                                   int64_t i, int d, bool cosine, const float* qs,
+                                   const uint32_t* cand, float* dist, int m) {
+    const int lane = threadIdx.x & 31;
+    auto add = [&](float& acc, float x, float y) {
+        if (cosine) {
+            acc = __fadd_rn(acc, __fmul_rn(x, y));
+        } else {
+            const float df = __fsub_rn(x, y);
+            acc = __fadd_rn(acc, __fmul_rn(df, df));
+        }
+    };
+    if (d < 64) {
+        for (int c = lane; c < m; c += 32) {
+            const int64_t j = cand[c];
+            float sum = 0.0f;
+            for (int t = 0; t < d; ++t) add(sum, qs[t], __ldg(X + j * d + t));
+            dist[c] = dense_distance(sum, norms, i, j, cosine);
+        }
+        return;
+    }
+    const int g = lane >> 3, r = lane & 7, leader = lane & ~7;
+    const int body = (d / 8) * 8;
+    for (int base = 0; base < m; base += 4) {
+        const int c = base + g;
+        const bool act = c < m;
+        const int64_t j = act ? static_cast<int64_t>(cand[c]) : i;
+        const float* y = X + j * d;
+        float acc = 0.0f;
+        for (int t = r; t < body; t += 8) add(acc, qs[t], __ldg(y + t));
+        float sum = __shfl_sync(0xffffffffu, acc, leader);
+#pragma unroll
+        for (int l = 1; l < 8; ++l) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, acc, leader + l));
+        if (r == 0 && act) {
+            for (int t = body; t < d; ++t) add(sum, qs[t], y[t]);
+            dist[c] = dense_distance(sum, norms, i, j, cosine);
+        }
+    }
+}
+
+// Distances of the query row (in shared memory) to the candidate rows
+// cand[0, m).  d a multiple of four and 16-byte aligned rows: from 64 columns on
+// two lanes share a candidate, lane half h holding the reference's AVX2
+// lanes 4h to 4h + 3 of 16-byte loads; below, one lane takes a candidate.
+// Same operations in the same order as eval_candidates.
+__device__ inline void eval_quads(const float* __restrict__ X, const float* __restrict__ norms,
+                                  int64_t i, int d, bool cosine, const float* qs,
+                                  const uint32_t* cand, float* dist, int m) {
+    const int lane = threadIdx.x & 31;
+    const float4* q4 = reinterpret_cast<const float4*>(qs);
+    auto add = [&](float& acc, float x, float y) {
+        if (cosine) {
+            acc = __fadd_rn(acc, __fmul_rn(x, y));
+        } else {
+            const float df = __fsub_rn(x, y);
+            acc = __fadd_rn(acc, __fmul_rn(df, df));
+        }
+    };
+    if (d < 64) {
+        for (int c = lane; c < m; c += 32) {
+            const int64_t j = cand[c];
+            const float4* y4 = reinterpret_cast<const float4*>(X + j * d);
+            float sum = 0.0f;
+#pragma unroll 4
+            for (int t = 0; t < d / 4; ++t) {
+                const float4 y = __ldg(y4 + t), x = q4[t];
+                add(sum, x.x, y.x);
+                add(sum, x.y, y.y);
+                add(sum, x.z, y.z);
+                add(sum, x.w, y.w);
+            }
+            dist[c] = dense_distance(sum, norms, i, j, cosine);
+        }
+        return;
+    }
+    const int half = lane & 1, steps = d / 8;
+    for (int base = 0; base < m; base += 16) {
+        const int c = base + (lane >> 1);
+        const int64_t j = c < m ? static_cast<int64_t>(cand[c]) : i;
+        const float4* y4 = reinterpret_cast<const float4*>(X + j * d) + half;
+        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+#pragma unroll 4
+        for (int t = 0; t < steps; ++t) {
+            const float4 y = __ldg(y4 + 2 * t), x = q4[2 * t + half];
+            add(a0, x.x, y.x);
+            add(a1, x.y, y.y);
+            add(a2, x.z, y.z);
+            add(a3, x.w, y.w);
+        }
+        // lanes 0 to 3 summed in order, handed on, then 4 to 7 and the tail
+        float sum = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
+        sum = __shfl_sync(0xffffffffu, sum, lane & ~1);
+        if (half == 1 && c < m) {
+            sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, a0), a1), a2), a3);
+            for (int t = steps * 8; t < d; ++t) add(sum, qs[t], X[j * d + t]);
+            dist[c] = dense_distance(sum, norms, i, j, cosine);
+        }
+    }
+}
+
+template <bool SP>
+__host__ __device__ inline size_t nd_reg_smem(int cap, int d) {
+    return static_cast<size_t>(cap) * 8 + static_cast<size_t>((d + 3) / 4) * 16 * (SP ? 2 : 1);
+}
+
+template <bool SP, int NPL>
+__global__ void __launch_bounds__(kWarps * 32) nd_iter_reg_kernel(NdArgs p, uint64_t iteration) {
+    constexpr int kCap = 32 * NPL;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int row_words = SP ? p.csr.max_nnz : p.d;
+    unsigned char* ws = smem + warp * nd_reg_smem<SP>(kCap, row_words);
+    float* qs = reinterpret_cast<float*>(ws);
+    uint32_t* cand = reinterpret_cast<uint32_t*>(ws + static_cast<size_t>((row_words + 3) / 4) * 16 *
+                                                          (SP ? 2 : 1));
+    float* dist = reinterpret_cast<float*>(cand + kCap);
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * kWarps + warp;
+    if (i >= p.n) return;
+    const int qn = load_query<SP>(p, i, qs);
+    const int k = p.k;
+    const uint64_t rbase = iteration << 40;
+    // neighbours, their neighbours, the row itself, random rows
+    uint32_t v[NPL];
+    const int32_t own = lane < k ? p.old_idx[i * k + lane] : 0;
+    const int base2 = k + k * k;
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) {
+        const int t = r * 32 + lane;  // any placement: the values are sorted next
+        const int t2 = t - k;
+        const int32_t nb = __shfl_sync(0xffffffffu, own, t < k ? t : (t2 / k) & 31);
+        uint32_t x = ~0u;
+        if (t < k)
+            x = static_cast<uint32_t>(nb);
+        else if (t < base2)
+            x = static_cast<uint32_t>(p.old_idx[static_cast<int64_t>(nb) * k + t2 % k]);
+        else if (t == base2)
+            x = static_cast<uint32_t>(i);
+        else if (t <= base2 + p.expl)
+            x = rng_below(rng_word(p.seed, static_cast<uint64_t>(i),
+                                   rbase + static_cast<uint64_t>(t - base2 - 1)),
+                          static_cast<uint32_t>(p.n));
+        v[r] = x;
+    }
+    reg_sort_u32<NPL>(v);
+    // unique, in ascending order
+    uint32_t prev = __shfl_up_sync(0xffffffffu, v[NPL - 1], 1);
+    if (lane == 0) prev = ~0u;
+    int mine = 0;
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) {
+        const uint32_t before = r == 0 ? prev : v[r - 1];
+        mine += v[r] != ~0u && v[r] != before;
+    }
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += u;
+    }
+    const int uniq = __shfl_sync(0xffffffffu, at, 31);
+    at -= mine;
+#pragma unroll
+    for (int r = 0; r < NPL; ++r) {
+        const uint32_t before = r == 0 ? prev : v[r - 1];
+        if (v[r] != ~0u && v[r] != before) cand[at++] = v[r];
+    }
+    __syncwarp();
+    // Random partial Fisher-Yates down to max_candidates (lib.rs:3076-3083).
+    // Swap s exchanges positions s and r_s >= s, so position s holds its final
+    // element from then on and position r_s receives what stood at s.  The
+    // element that ends at a position p that is cut off therefore came there
+    // with the last swap s with r_s = p, which took it from position s, where
+    // the last swap before s with r = s had put it, and so on: `last` holds
+    // those swaps, and a lane follows the chain of each position cut off.
+    int m = uniq;
+    if (uniq > p.maxc) {
+        int* last = reinterpret_cast<int*>(dist);
+        for (int c = lane; c < uniq; c += 32) last[c] = -1;
+        __syncwarp();
+        for (int s = lane; s < p.maxc; s += 32) {
+            const int r = s + static_cast<int>(rng_below(
+                                  rng_word(p.seed, static_cast<uint64_t>(i),
+                                           rbase + (1u << 20) + static_cast<uint64_t>(s)),
+                                  static_cast<uint32_t>(uniq - s)));
+            if (r != s) atomicMax(&last[r], s);
+        }
+        __syncwarp();
+        for (int c = p.maxc + lane; c < uniq; c += 32) {
+            int e = c;
+            for (int s = last[c]; s >= 0; s = last[s]) e = s;
+            cand[e] |= 0x80000000u;  // cut off
+        }
+        __syncwarp();
+        m = 0;
+        for (int base = 0; base < uniq; base += 32) {
+            const int c = base + lane;
+            const uint32_t x = c < uniq ? cand[c] : ~0u;
+            const bool keep = (x & 0x80000000u) == 0;
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            __syncwarp();
+            if (keep) cand[m + __popc(mask & ((1u << lane) - 1))] = x;
+            __syncwarp();
+            m += __popc(mask);
+        }
+    }
+    if constexpr (SP) {
+        for (int c = lane; c < m; c += 32)
+            dist[c] = csr_distance(p.csr, i, cand[c], p.metric, reinterpret_cast<const int32_t*>(qs),
+                                   qs + p.csr.max_nnz, qn);
+    } else if (p.quads) {
+        eval_quads(p.X, p.norms, i, p.d, p.cosine, qs, cand, dist, m);
+    } else {
+        eval_scalar(p.X, p.norms, i, p.d, p.cosine, qs, cand, dist, m);
+    }
+    __syncwarp();
+    if (lane == 0)
+        atomicAdd(p.evaluated + blockIdx.x % kEvalSlots, static_cast<unsigned long long>(m));
+    // the 32 best keys, sorted across the lanes
+    uint64_t best = ~0ull;
+    for (int base = 0; base < m; base += 32) {
+        const int c = base + lane;
+        uint64_t key = c < m ? knn_key(dist[c], cand[c]) : ~0ull;
+        const uint64_t worst = __shfl_sync(0xffffffffu, best, k - 1);
+        unsigned in = __ballot_sync(0xffffffffu, key < worst);
+        if (__popc(in) > kInsertMost) {
+            best = merge_best(best, key);
+        } else {
+            while (in) {
+                const int b = __ffs(in) - 1;
+                in &= in - 1;
+                const uint64_t x = __shfl_sync(0xffffffffu, key, b);
+                const int pos = __popc(__ballot_sync(0xffffffffu, best < x));
+                const uint64_t up = __shfl_up_sync(0xffffffffu, best, 1);
+                if (lane > pos)
+                    best = up;
+                else if (lane == pos)
+                    best = x;
+            }
+        }
+    }
+    bool diff = false;
+    if (lane < k) {
+        const int32_t ni = static_cast<int32_t>(key_index(best));
+        const float nd = key_dist(best);
+        diff = ni != own || nd != p.old_dist[i * k + lane];
+        p.new_idx[i * k + lane] = ni;
+        p.new_dist[i * k + lane] = nd;
+    }
+    if (__any_sync(0xffffffffu, diff) && lane == 0) *p.changed = 1;
+}
+
 }  // namespace
 
 namespace {
@@ -398,10 +703,26 @@ int64_t nndescent_run(NdArgs p, int64_t n, int k, int64_t n_iters, size_t smem, 
     UMAPB_CUDA(cudaFuncSetAttribute(nd_init_kernel<SP>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
-    UMAPB_CUDA(cudaFuncSetAttribute(nd_iter_kernel<SP>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
     const unsigned grid = static_cast<unsigned>(ceil_div(n, kWarps));
+    // k <= 31 keeps the candidates in registers (row indices below 2^31, k
+    // best within one warp's list); longer lists take the shared-memory form
+    void (*iterate)(NdArgs, uint64_t) = nd_iter_kernel<SP>;
+    size_t iter_smem = smem;
+    if (k <= 31) {
+        switch (p.cap / 32) {
+            case 1: iterate = nd_iter_reg_kernel<SP, 1>; break;
+            case 2: iterate = nd_iter_reg_kernel<SP, 2>; break;
+            case 4: iterate = nd_iter_reg_kernel<SP, 4>; break;
+            case 8: iterate = nd_iter_reg_kernel<SP, 8>; break;
+            case 16: iterate = nd_iter_reg_kernel<SP, 16>; break;
+            case 32: iterate = nd_iter_reg_kernel<SP, 32>; break;
+            default: break;
+        }
+        if (iterate != nd_iter_kernel<SP>)
+            iter_smem = kWarps * nd_reg_smem<SP>(p.cap, SP ? p.csr.max_nnz : p.d);
+    }
+    UMAPB_CUDA(cudaFuncSetAttribute(iterate, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    static_cast<int>(iter_smem)));
     int32_t* cur_i = out_idx;
     float* cur_d = out_dist;
     int32_t* nxt_i = idx_b.get();
@@ -430,7 +751,7 @@ int64_t nndescent_run(NdArgs p, int64_t n, int k, int64_t n_iters, size_t smem, 
         p.new_idx = nxt_i;
         p.new_dist = nxt_d;
         UMAPB_CUDA(cudaEventRecord(e0, s));
-        nd_iter_kernel<SP><<<grid, kWarps * 32, smem, s>>>(p, static_cast<uint64_t>(it + 1));
+        iterate<<<grid, kWarps * 32, iter_smem, s>>>(p, static_cast<uint64_t>(it + 1));
         UMAPB_LAUNCH_CHECK();
         UMAPB_CUDA(cudaEventRecord(e1, s));
         std::swap(cur_i, nxt_i);
@@ -500,6 +821,7 @@ int64_t nndescent(const float* X, int64_t n, int d, int k, int metric, int64_t c
     p.k = k;
     p.cosine = metric == UMAPB_METRIC_COSINE;
     p.metric = metric;
+    p.quads = d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     p.seed = seed;
     return nndescent_run<false>(p, n, k, n_iters, smem, out_idx, out_dist, s, stats);
 }
