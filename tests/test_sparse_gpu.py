@@ -278,3 +278,26 @@ def test_sparse_fit_takes_nndescent_on_explicit_approximate_request():
     te = diagnostics.quality(dense, exact, sample=None)["trustworthiness"]
     print("trust approximate", ta, "exact", te)
     assert np.all(np.isfinite(emb)) and abs(ta - te) <= 0.02
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+def test_sparse_knn_at_the_edges_of_the_far_row_test(orc, metric):
+    # rows are turned away before their distance is computed once the list is
+    # full: duplicates and zero distances at the list's end, empty rows, norms
+    # from 1e-21 to 1e18, dots that cancel to 0 (norms that overflow give the
+    # cosine distance NaN, whose place among the others is not defined)
+    rng = np.random.default_rng(0)
+    x = rng.normal(size=(2500, 40)).astype(np.float32)
+    x[x < 0.3] = 0
+    x[5] = x[9] = 0
+    x[100:150] = x[100]
+    x[200:203] *= np.float32(1e18)
+    x[203:206] *= np.float32(1e-21)
+    x[210, :] = 0
+    x[210, :2] = (1, -1)
+    x[211, :] = 0
+    x[211, :2] = (1, 1)
+    m = sp.csr_matrix(x)
+    gi, gd = _gpu_knn(m, 20, metric)
+    oi, od = orc.csr_knn(m, 20, metric)
+    assert np.array_equal(gi, oi) and np.array_equal(gd, od, equal_nan=True)

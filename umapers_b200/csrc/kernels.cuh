@@ -82,9 +82,8 @@ void csr_from_dense(const float* X, int64_t n, int64_t d, CsrDevice& out, cudaSt
 // (squared norm, index).
 struct CsrIndex {
     int64_t n_tiles = 0;
-    DevBuf<int64_t> tile_colptr;  // n_tiles * n_cols + 1 offsets
-    DevBuf<int32_t> tile_rows;    // row within its tile
-    DevBuf<float> tile_vals;
+    DevBuf<int32_t> tile_colptr;  // n_tiles * n_cols + 1 offsets
+    DevBuf<uint2> tile_entries;   // row within its tile, value bits
     DevBuf<int32_t> norm_order;
 };
 void csr_index(const CsrDevice& r, CsrIndex& out, cudaStream_t s);
