@@ -257,3 +257,28 @@ def test_tensor_knn_pixel_like_rows_784(orc):
     rows = rng.choice(6000, 40, replace=False)
     oi, od = orc.exact_knn_rows(x, rows, 15)
     np.testing.assert_array_equal(ti[rows], oi)
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+@pytest.mark.parametrize("nq,n,d,k", [
+    (1, 1, 64, 1), (3, 63, 64, 1), (5, 64, 68, 31), (130, 65, 66, 32), (7, 129, 40, 33),
+    (0, 257, 72, 62), (0, 700, 100, 15), (0, 1500, 65, 32), (300, 2500, 128, 15), (2, 40000, 96, 20),
+    (0, 4000, 200, 62)])
+def test_lists_and_rerank_at_their_edges(metric, nq, n, d, k):
+    # lists that stay empty, hold fewer than 32 keys, or are merged with at most
+    # 32 and with more appended keys; one to many candidate splits; re-ranked
+    # rows of whole quads and not, from 64 columns and below, k on both sides of
+    # 32: bit for bit as the plain path
+    x = workloads.isotropic_mixture(n, d, 3, 2.0, seed=n + d)
+    if n > 100:
+        x[n // 2: n // 2 + 40] = x[3]  # ties within and beyond a list
+    if nq:
+        q = workloads.isotropic_mixture(nq, d, 3, 2.0, seed=n + d + 1)
+        q[0] = x[0]
+        a = gu.knn_query(q, x, k, metric, "tensor")
+        b = gu.knn_query(q, x, k, metric, "plain")
+    else:
+        a = gu.knn_exact(x, k, metric, "tensor")
+        b = gu.knn_exact(x, k, metric, "plain")
+    assert np.array_equal(a[0], b[0])
+    assert np.array_equal(a[1].view(np.uint32), b[1].view(np.uint32))

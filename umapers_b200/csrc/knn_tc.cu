@@ -270,10 +270,6 @@ __device__ __forceinline__ T rank_of(T lo, T hi, int r) {
     return r < 32 ? a : b;
 }
 
-// Held keys at or above this count are merged in one bitonic pass instead of
-// key by key (about 6 sequential insertions cost as much).
-constexpr int kBulkMergeMin = 6;
-
 // A list occupies LS slots: its S smallest keys so far, sorted ascending
 // (order-mapped L << 32 | index), then up to HC keys appended unsorted since
 // the last merge, each below that merge's threshold and stored with L as raw
@@ -283,41 +279,65 @@ __device__ __forceinline__ uint64_t held_key(uint64_t raw) {
            static_cast<uint32_t>(raw);
 }
 
-// Merges the `held` appended keys (at most HC) into the sorted ones, one key
-// per lane, and returns the new S-th smallest L, or +inf while the list holds
-// fewer than S keys.
-__device__ __forceinline__ float merge_held(uint64_t* lst, int held) {
+// Merges order keys by their slot in the list and the leading bits of L: the
+// low kSlotBits bits of the order-mapped L give way to the slot, so 32-bit
+// words are sorted instead of 64-bit keys.  A list then keeps 32 keys such
+// that every key left out has an L of at least the largest kept one's with
+// those bits cleared; the threshold and the re-rank's bound are taken from
+// that (2^-16 of L, far inside the slack of the error bound).  The kernel on
+// 300,000 queries of 8,000 x 128 rows, whose short walks are mostly merges,
+// 6.9 -> 6.0 ms; 1M x 64 199.9 -> 194.7.  What is left there is the appends: with
+// 32 rows a warp, some row is pending in most tiles.
+constexpr int kSlotBits = 7;
+constexpr uint32_t kSlotMask = (1u << kSlotBits) - 1u;
+static_assert(LS < (1 << kSlotBits), "a slot fits its bits, with one value left over");
+__device__ __forceinline__ uint32_t slot_word(uint64_t key, int slot) {
+    return key == ~0ull ? ~0u : (static_cast<uint32_t>(key >> 32) & ~kSlotMask) | slot;
+}
+
+// Merges the `held` appended keys (at most HC) into the sorted ones (none
+// yet in a `fresh` list, whose slots were never written), one key per lane,
+// and returns the new threshold, or +inf while the list holds fewer than S
+// keys.
+__device__ __forceinline__ float merge_held(uint64_t* lst, int held, bool fresh) {
     const int lane = threadIdx.x & 31;
     __syncwarp();  // the appended keys were stored by other lanes
-    uint64_t lk = lst[lane];
-    uint64_t h0 = lane < held ? held_key(lst[S + lane]) : ~0ull;
-    uint64_t h1 = lane + 32 < held ? held_key(lst[S + 32 + lane]) : ~0ull;
+    const uint64_t lk = fresh ? ~0ull : lst[lane];
+    const uint64_t h0 = lane < held ? held_key(lst[S + lane]) : ~0ull;
+    uint64_t h1 = ~0ull;
+    uint32_t w = slot_word(h0, S + lane);
     if (held > 32) {
-        // both halves sorted at once; the 32 smallest of them (lane-wise min
-        // of one and the other reversed, a bitonic sequence), sorted, then
-        // merged with the list the same way
-        warp_sort_asc2<uint64_t>(h0, h1);
-        const uint64_t r1 = __shfl_sync(0xffffffffu, h1, 31 - lane);
-        const uint64_t m = warp_bitonic_sort<uint64_t>(h0 < r1 ? h0 : r1);
-        const uint64_t rm = __shfl_sync(0xffffffffu, m, 31 - lane);
-        lk = warp_bitonic_sort<uint64_t>(lk < rm ? lk : rm);
-    } else if (held >= kBulkMergeMin) {
-        lk = warp_merge_keys(lk, h0);
+        // both halves sorted at once; the 32 smallest of them are the lane-wise
+        // minima of one and the other reversed, a bitonic sequence
+        if (lane + 32 < held) h1 = held_key(lst[S + 32 + lane]);
+        uint32_t w1 = slot_word(h1, S + 32 + lane);
+        warp_sort_asc2<uint32_t>(w, w1);
+        w = warp_bitonic_sort<uint32_t>(min(w, __shfl_sync(0xffffffffu, w1, 31 - lane)));
     } else {
-        for (int b = 0; b < held; ++b) {
-            const uint64_t key = __shfl_sync(0xffffffffu, h0, b);
-            const int pos = __popc(__ballot_sync(0xffffffffu, lk < key));
-            const uint64_t up = __shfl_up_sync(0xffffffffu, lk, 1);
-            if (lane > pos)
-                lk = up;
-            else if (lane == pos)
-                lk = key;
-        }
+        w = warp_sort_asc<uint32_t>(w);
     }
-    lst[lane] = lk;
+    w = warp_bitonic_sort<uint32_t>(
+        min(slot_word(lk, lane), __shfl_sync(0xffffffffu, w, 31 - lane)));
+    // the keys the sorted words stand for
+    const int slot = static_cast<int>(w & kSlotMask);
+    uint64_t key = __shfl_sync(0xffffffffu, lk, slot & 31);
+    const uint64_t from0 = __shfl_sync(0xffffffffu, h0, slot & 31);
+    if (slot >= 32) key = from0;
+    if (held > 32) {
+        const uint64_t from1 = __shfl_sync(0xffffffffu, h1, slot & 31);
+        if (slot >= 64) key = from1;
+    }
+    lst[lane] = w == ~0u ? ~0ull : key;
     __syncwarp();
-    const uint64_t last = __shfl_sync(0xffffffffu, lk, S - 1);
-    return last == ~0ull ? INFINITY : o2f(static_cast<uint32_t>(last >> 32));
+    const uint32_t last = __shfl_sync(0xffffffffu, w, S - 1);
+    return last == ~0u ? INFINITY : o2f(last & ~kSlotMask);
+}
+
+// Brings a list's lines to L1 ahead of its merge.
+__device__ __forceinline__ void prefetch_list(const uint64_t* lst) {
+    const int lane = threadIdx.x & 31;
+    if (lane * 16 < LS)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(lst + lane * 16));
 }
 
 // Appends, for one lane's row, its values below t (columns below lim) as
@@ -355,7 +375,7 @@ struct TcArgs {
     int64_t n_ctiles;     // candidate tiles
     uint64_t* lists;      // n_q x n_split x (BN / 64) lists of LS slots of keys (L
                           // order-mapped << 32 | index), one list per (row, candidate split,
-                          // 64-column group)
+                          // 64-column group); the kernel writes every list
     const int32_t* start_tile;  // per query group, the first candidate tile to visit (rows in
                                 // cell order, one split), or null for the staggered start
     int* err;
@@ -427,6 +447,7 @@ __device__ __forceinline__ bool tc_epilogue(const TcArgs& p, int warp, int lane,
         };
         float tau = INFINITY;  // this row's list: its S-th smallest key at the last merge
         int held = 0;          // keys appended behind the sorted ones since then
+        bool fresh = row_ok;   // nothing merged yet: the sorted slots are unwritten
         for (int32_t c = 0; c < w.len; ++c, ++cg) {
             const uint32_t buf = static_cast<uint32_t>(cg & 1);
             const uint32_t par = static_cast<uint32_t>((cg >> 1) & 1);
@@ -466,11 +487,14 @@ __device__ __forceinline__ bool tc_epilogue(const TcArgs& p, int warp, int lane,
             while (over) {
                 const int cur = __ffs(over) - 1;
                 over &= over - 1;
+                if (over) prefetch_list(list_of(__shfl_sync(0xffffffffu, row, __ffs(over) - 1)));
                 const float nt = merge_held(list_of(__shfl_sync(0xffffffffu, row, cur)),
-                                            __shfl_sync(0xffffffffu, held, cur));
+                                            __shfl_sync(0xffffffffu, held, cur),
+                                            __shfl_sync(0xffffffffu, fresh, cur));
                 if (lane == cur) {
                     tau = nt;
                     held = 0;
+                    fresh = false;
                 }
             }
             t = mine ? tau : -INFINITY;
@@ -479,13 +503,15 @@ __device__ __forceinline__ bool tc_epilogue(const TcArgs& p, int warp, int lane,
                        : append_row<false>(r, t, valid_cols, colh, dst, held);
         }
         if (!ok) break;
-        // every list of the unit ends sorted, with nothing held
-        unsigned rest = __ballot_sync(0xffffffffu, held > 0);
+        // every list of the unit ends written and sorted, with nothing held
+        unsigned rest = __ballot_sync(0xffffffffu, held > 0 || fresh);
         while (rest) {
             const int cur = __ffs(rest) - 1;
             rest &= rest - 1;
+            if (rest) prefetch_list(list_of(__shfl_sync(0xffffffffu, row, __ffs(rest) - 1)));
             merge_held(list_of(__shfl_sync(0xffffffffu, row, cur)),
-                       __shfl_sync(0xffffffffu, held, cur));
+                       __shfl_sync(0xffffffffu, held, cur),
+                       __shfl_sync(0xffffffffu, fresh, cur));
         }
     }
     return ok;
@@ -911,6 +937,7 @@ struct RerankArgs {
     int d, k;
     double c, c0;
     bool cosine;
+    bool quads;            // rows of whole, aligned 16-byte quads, 64 columns or more
     const ScaleInfo* sc;
     const int32_t* omap;   // query position -> output row (null: identity)
     const int32_t* rmap;   // candidate position -> original index (null: identity)
@@ -918,9 +945,66 @@ struct RerankArgs {
     float* out_dist;
     int* fb_count;
     int32_t* fb_rows;      // output rows that could not be certified
+    const int* err;        // the list kernel's error word: its lists are not read when set
 };
 
-__global__ void rerank_kernel(RerankArgs a) {
+constexpr int kRerankWarps = 8;
+
+// Exact FP32 squared distances (cosine: dot products) in the reference's
+// order of query row q to the rows buf[0, cnt), cnt <= 32, lane c returning
+// candidate c's.  Rows of whole, aligned 16-byte quads from 64 columns on:
+// two lanes share a candidate, lane half h adding the reference's AVX2 lanes
+// 4h to 4h + 3, so a warp's load covers whole 32-byte sectors of 16 rows.  The
+// re-rank of 300,000 rows of 128 columns 2.0 -> 1.4 ms (one lane a candidate,
+// list by list, before), of 60,013 cosine rows of 100 columns 1.2 -> 0.5.
+__device__ __forceinline__ float exact_values(const float* __restrict__ R, const float* __restrict__ q,
+                                              int d, bool cosine, bool quads, const uint32_t* buf,
+                                              int cnt) {
+    const int lane = threadIdx.x & 31;
+    if (!quads) {
+        if (lane >= cnt) return 0.0f;
+        const float* y = R + static_cast<int64_t>(buf[lane]) * d;
+        return cosine ? dot_ref(q, y, d) : sqdist_ref(q, y, d);
+    }
+    const int half = lane & 1, steps = d / 8;
+    const float4* q4 = reinterpret_cast<const float4*>(q) + half;
+    auto add = [&](float& acc, float x, float y) {
+        if (cosine) {
+            acc = __fadd_rn(acc, __fmul_rn(x, y));
+        } else {
+            const float df = __fsub_rn(x, y);
+            acc = __fadd_rn(acc, __fmul_rn(df, df));
+        }
+    };
+    float mine = 0.0f;
+    for (int base = 0; base < cnt; base += 16) {
+        const int c = min(base + (lane >> 1), cnt - 1);
+        const float* y = R + static_cast<int64_t>(buf[c]) * d;
+        const float4* y4 = reinterpret_cast<const float4*>(y) + half;
+        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+#pragma unroll 4
+        for (int t = 0; t < steps; ++t) {
+            const float4 v = __ldg(y4 + 2 * t), x = __ldg(q4 + 2 * t);
+            add(a0, x.x, v.x);
+            add(a1, x.y, v.y);
+            add(a2, x.z, v.z);
+            add(a3, x.w, v.w);
+        }
+        // lanes 0 to 3 summed in order, handed on, then 4 to 7 and the tail
+        float sum = __fadd_rn(__fadd_rn(__fadd_rn(a0, a1), a2), a3);
+        sum = __shfl_sync(0xffffffffu, sum, lane & ~1);
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, a0), a1), a2), a3);
+        if (half == 1)
+            for (int t = steps * 8; t < d; ++t) add(sum, q[t], y[t]);
+        const float got = __shfl_sync(0xffffffffu, sum, 2 * (lane & 15) + 1);
+        if ((lane & 16) == base) mine = got;
+    }
+    return mine;
+}
+
+__global__ void __launch_bounds__(kRerankWarps * 32) rerank_kernel(RerankArgs a) {
+    __shared__ uint32_t cands[kRerankWarps][64];
+    if (*a.err != 0) return;  // the lists may be unwritten; the host reports the error
     const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= a.n_q) return;
@@ -928,8 +1012,9 @@ __global__ void rerank_kernel(RerankArgs a) {
     const int64_t orow = a.omap != nullptr ? a.omap[row] : row;
     const uint64_t* rl = a.lists + row * a.n_lists * LS;
     // The smallest bound a candidate missing from every list can have: a full
-    // list left out only candidates with L >= its largest entry, a list that
-    // is not full kept every candidate of its range.
+    // list left out only candidates with L at or above its largest entry's with
+    // the slot bits cleared, a list that is not full kept every candidate of
+    // its range.
     double bound = INFINITY;
     for (int h = 0; h < a.n_lists; ++h) {
         const uint64_t lk = rl[h * LS + lane];
@@ -938,7 +1023,7 @@ __global__ void rerank_kernel(RerankArgs a) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
         if (__popc(__ballot_sync(0xffffffffu, valid)) == S)
-            bound = fmin(bound, static_cast<double>(lmax));
+            bound = fmin(bound, static_cast<double>(o2f(f2o(lmax) & ~kSlotMask)));
     }
     // Upper bounds U = L + 2e (rounded up to FP32): `below` counts the
     // candidates with U < bound (k of them certify the row), and T is the k-th
@@ -953,7 +1038,8 @@ __global__ void rerank_kernel(RerankArgs a) {
     const bool wide = k > 32;
     for (int h = 0; h < a.n_lists; ++h) {
         const uint64_t lk = rl[h * LS + lane];
-        const float l0 = o2f(static_cast<uint32_t>(__shfl_sync(0xffffffffu, lk, 0) >> 32));
+        // at or below every L of the list (an empty list: NaN, never below T)
+        const float l0 = o2f(static_cast<uint32_t>(__shfl_sync(0xffffffffu, lk, 0) >> 32) & ~kSlotMask);
         double U = INFINITY;
         if (lk != ~0ull) {
             const double nc =
@@ -975,30 +1061,45 @@ __global__ void rerank_kernel(RerankArgs a) {
         }
     }
     const float T = rank_of<float>(topu, topu_hi, k - 1);
-    // Exact keys in the reference's order for the candidates with L <= T; the
-    // 32 (k <= 32) or 64 smallest are kept sorted across the warp (bitonic
-    // merge of each list's keys into them).
+    // Exact keys in the reference's order for the candidates with L <= T,
+    // gathered from all lists 32 at a time; the 32 (k <= 32) or 64 smallest
+    // are kept sorted across the warp.
     const float* qrow = a.Q + row * d;
     const float qn = a.cosine ? __fsqrt_rn(a.qsq[row]) : 0.0f;
+    uint32_t* buf = cands[threadIdx.x >> 5];
     uint64_t top = ~0ull, top_hi = ~0ull;
-    for (int h = 0; h < a.n_lists; ++h) {
-        const uint64_t lk = rl[h * LS + lane];
-        const bool take = lk != ~0ull && o2f(static_cast<uint32_t>(lk >> 32)) <= T;
-        if (__ballot_sync(0xffffffffu, take) == 0) continue;
+    int have = 0;
+    auto flush = [&](int cnt) {
+        __syncwarp();
+        const float v = exact_values(a.R, qrow, d, a.cosine, a.quads, buf, cnt);
         uint64_t key = ~0ull;
-        if (take) {
-            const uint32_t j = static_cast<uint32_t>(lk);
-            const float* crow = a.R + static_cast<int64_t>(j) * d;
-            const float dist = a.cosine
-                                   ? cosine_ref(dot_ref(qrow, crow, d), qn, __fsqrt_rn(a.rsq[j]))
-                                   : sqdist_ref(qrow, crow, d);
+        if (lane < cnt) {
+            const uint32_t j = buf[lane];
+            const float dist = a.cosine ? cosine_ref(v, qn, __fsqrt_rn(a.rsq[j])) : v;
             key = knn_key(dist, a.rmap != nullptr ? static_cast<uint32_t>(a.rmap[j]) : j);
         }
         if (wide)
             warp_merge64<uint64_t>(top, top_hi, key);
         else
             top = warp_merge_keys(top, key);
+    };
+    for (int h = 0; h < a.n_lists; ++h) {
+        const uint64_t lk = rl[h * LS + lane];
+        const bool take = lk != ~0ull && o2f(static_cast<uint32_t>(lk >> 32)) <= T;
+        const unsigned m = __ballot_sync(0xffffffffu, take);
+        if (m == 0) continue;
+        if (take) buf[have + __popc(m & ((1u << lane) - 1u))] = static_cast<uint32_t>(lk);
+        have += __popc(m);
+        if (have >= 32) {
+            flush(32);
+            have -= 32;
+            __syncwarp();
+            const uint32_t left = lane < have ? buf[32 + lane] : 0u;
+            __syncwarp();
+            if (lane < have) buf[lane] = left;
+        }
     }
+    if (have > 0) flush(have);
     // A zero cosine query has distance 0 to zero rows and 1 to the rest, which
     // its bound (built for unit rows) does not cover: it goes to the plain path.
     const bool failed = below < k || (a.cosine && a.qsq[row] == 0.0f);
@@ -1321,16 +1422,12 @@ void launch_max_sq(const float* sq, int64_t n, unsigned* out, cudaStream_t s) {
     UMAPB_LAUNCH_CHECK();
 }
 
-// Empties `count` lists: their S sorted slots become ~0 (the appended slots
-// are only read below the count a list holds).
-void clear_lists(uint64_t* lists, size_t count, cudaStream_t s) {
-    if (count == 0) return;
-    UMAPB_CUDA(cudaMemset2DAsync(lists, LS * sizeof(uint64_t), 0xFF, S * sizeof(uint64_t), count,
-                                 s));
-}
-
 void launch_rerank(const RerankArgs& ra, cudaStream_t s) {
-    rerank_kernel<<<static_cast<unsigned>(ceil_div(ra.n_q * 32, 256)), 256, 0, s>>>(ra);
+    RerankArgs a = ra;
+    a.quads = a.d >= 64 && a.d % 4 == 0 &&
+              ((reinterpret_cast<uintptr_t>(a.Q) | reinterpret_cast<uintptr_t>(a.R)) & 15) == 0;
+    rerank_kernel<<<static_cast<unsigned>(ceil_div(a.n_q, static_cast<int64_t>(kRerankWarps))),
+                    kRerankWarps * 32, 0, s>>>(a);
     UMAPB_LAUNCH_CHECK();
 }
 
@@ -1413,7 +1510,6 @@ void knn_tc(const float* Q, int64_t n_q, const float* R, int64_t n_r, int d, int
     launch_prep(R, rsq_p, n_r, d, g, sc.get(), bd, cosine, false, B.get(), s);
     const int n_lists = sh.lists() * a.n_split;
     DevBuf<uint64_t> lists(static_cast<size_t>(n_q) * n_lists * LS, s);
-    clear_lists(lists.get(), static_cast<size_t>(n_q) * n_lists, s);
     const SideMaps ma = side_maps(A.get(), n_q, g, sh, BM);
     const SideMaps mb = side_maps(B.get(), n_r, g, sh, sh.bn);
     a.lists = lists.get();
@@ -1441,6 +1537,7 @@ void knn_tc(const float* Q, int64_t n_q, const float* R, int64_t n_r, int d, int
     ra.rmap = perm;
     ra.out_idx = out_idx;
     ra.out_dist = out_dist;
+    ra.err = flags.get();
     ra.fb_count = flags.get() + 1;
     ra.fb_rows = fb_rows.get();
     launch_rerank(ra, s);
@@ -1485,7 +1582,6 @@ void knn_tc(const float* Q, int64_t n_q, const float* R, int64_t n_r, int d, int
         TcArgs a2 = plan(fb, n_r, g2, sh2, true, 2);
         const int n_lists2 = sh2.lists() * a2.n_split;
         DevBuf<uint64_t> lists2(static_cast<size_t>(fb) * n_lists2 * LS, s);
-        clear_lists(lists2.get(), static_cast<size_t>(fb) * n_lists2, s);
         const SideMaps ma2 = side_maps(A2.get(), fb, g2, sh2, BM);
         a2.lists = lists2.get();
         a2.err = flags.get() + 2;
@@ -1504,6 +1600,7 @@ void knn_tc(const float* Q, int64_t n_q, const float* R, int64_t n_r, int d, int
         rb.n_q = fb;
         rb.omap = fb_rows.get();
         rb.rmap = perm;
+        rb.err = flags.get() + 2;
         rb.fb_count = flags.get() + 3;
         rb.fb_rows = fb2_rows.get();
         launch_rerank(rb, s);
@@ -1625,9 +1722,8 @@ void knn_noalloc(const float* X, int64_t n, int d, int k, int32_t* out_idx, floa
     ScaleInfo* sc = reinterpret_cast<ScaleInfo*>(carve(sizeof(ScaleInfo)));
     int32_t* fb_rows = reinterpret_cast<int32_t*>(carve(static_cast<size_t>(n) * 4));
 
-    // every call starts from cleared shortlists and flags (the array keeps
-    // the previous call's contents)
-    clear_lists(lists, static_cast<size_t>(n) * sh.lists(), s);
+    // every call starts from cleared flags (the array keeps the previous
+    // call's contents); the kernel writes every shortlist
     UMAPB_CUDA(cudaMemsetAsync(flags, 0, 8 * sizeof(int), s));
     row_norms(X, n, d, nullptr, sq, s);
     unsigned* max_bits = reinterpret_cast<unsigned*>(flags + 4);
@@ -1658,6 +1754,7 @@ void knn_noalloc(const float* X, int64_t n, int d, int k, int32_t* out_idx, floa
     ra.sc = sc;
     ra.out_idx = out_idx;
     ra.out_dist = out_dist;
+    ra.err = flags;
     ra.fb_count = flags + 1;
     ra.fb_rows = fb_rows;
     launch_rerank(ra, s);
