@@ -106,3 +106,50 @@ def test_long_rows_give_the_dense_eigenvectors(dim):
     # N(0, 1e-4) noise on every coordinate (6 sigma), FP32 products (6e-8)
     # over eigenvalue gaps of 1e-3 at a scale of 10
     assert np.abs(g - ref).max() < 6e-4 + 10 * 6e-8 / 1e-3 * 2
+
+
+def equitable_graph(blocks, m, seed=11):
+    """A path of blocks of m nodes: six random m-cycles inside each block, node
+    i of a block tied to node i of the next.  Every node of a block has the same
+    weight to each block, so the leading eigenvectors of the normalised matrix
+    are constant on the blocks and come from the blocks x blocks quotient."""
+    rng = np.random.default_rng(seed)
+    h, t, w = [], [], []
+    tie = 0.3 + 0.17 * np.arange(blocks - 1)
+    for b in range(blocks):
+        for _ in range(6):
+            cyc = rng.permutation(m) + b * m
+            h.append(cyc), t.append(np.roll(cyc, 1)), w.append(np.full(m, 0.5))
+        if b + 1 < blocks:
+            i = np.arange(m) + b * m
+            h.append(i), t.append(i + m), w.append(np.full(m, tie[b]))
+    h, t, w = np.concatenate(h), np.concatenate(t), np.concatenate(w)
+    n = blocks * m
+    key, inv = np.unique(np.concatenate([h * n + t, t * n + h]), return_inverse=True)
+    weight = np.bincount(inv, np.concatenate([w, w])).astype(np.float32)
+    deg = 6.0 + np.append(tie, 0.0) + np.append(0.0, tie)
+    q = np.diag(6.0 / deg)
+    for b in range(blocks - 1):
+        q[b, b + 1] = q[b + 1, b] = tie[b] / np.sqrt(deg[b] * deg[b + 1])
+    return (key // n).astype(np.int32), (key % n).astype(np.int32), weight, q
+
+
+# one chunk of rows and one row more than it, a whole bundle of 16 chunks and
+# one more, more chunks than are split over CTAs, chunks of more than 1024 rows
+@pytest.mark.parametrize("dim,m", [(1, 342), (2, 256), (2, 257), (2, 4096), (2, 4097),
+                                   (3, 6001), (4, 341), (4, 25_271), (2, 38_001), (2, 77_003)])
+def test_orthonormalisation_at_its_chunk_edges(dim, m):
+    blocks = dim + 2
+    h, t, w, q = equitable_graph(blocks, m)
+    val, vec = np.linalg.eigh(q)
+    val = val[::-1]
+    assert np.min(-np.diff(val)) > 4e-3 and val[dim] > 0.7  # the cycles' bulk ends near 0.55
+    x = np.zeros((blocks * m, 16), np.float32)
+    g, used = gu.spectral_init(x, h, t, w, dim, 42)
+    assert used
+    ref = np.repeat(vec[:, ::-1][:, 1:dim + 1], m, axis=0)
+    ref = ref * 10.0 / np.abs(ref).max()
+    ref = ref * np.sign((ref * g).sum(0))
+    # N(0, 1e-4) noise on every coordinate (6 sigma), FP32 products (6e-8)
+    # over eigenvalue gaps of 4e-3 at a scale of 10
+    assert np.abs(g - ref).max() < 6e-4 + 10 * 6e-8 / 4e-3 * 2

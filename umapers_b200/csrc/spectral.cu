@@ -341,144 +341,102 @@ struct Chunk {
     int32_t slot;
     int32_t start;  // position range [start, end)
     int32_t end;
+    int32_t first;  // index of the slot's first chunk
+    int32_t of;     // chunks of the slot
+    int32_t bundle; // index of the slot's first bundle of kBundle chunks
 };
+constexpr int kBundle = 16;
 
-// Upper triangle of A^T B per slot over contiguous position ranges, FP64.
-// S is a multiple of 3 ((dim + 1) * 6), so the upper triangle is covered by
-// NT = T (T + 1) / 2 tiles of 3 x 3 entries (T = S / 3); thread t owns tile
-// t % NT for the rows t / NT, t / NT + G, ... of each staged slab (G row
-// groups).  Slabs of R rows are staged in shared memory as FP64, the next
-// slab's FP32 rows wait in registers meanwhile; at the end the G partial
-// tiles are summed in shared memory and added to G atomically.
+// Upper triangle of A^T B over a chunk's rows, FP64.  S is a multiple of 3
+// ((dim + 1) * 6), so the upper triangle is covered by NT = T (T + 1) / 2
+// tiles of 3 x 3 entries (T = S / 3).  The rows of a chunk are dealt to G
+// groups (row r of each slab of R rows to group r % G) and a thread keeps one
+// tile of one group; the groups' tiles are then added in order.
+constexpr int kOrthoThreads = 256;
+
 template <int S, int SP>
 struct GramShape {
     static_assert(S % 3 == 0, "the block width is a multiple of 3");
     static constexpr int T = S / 3;
     static constexpr int NT = T * (T + 1) / 2;
-    static constexpr int G = 256 / NT;
+    static constexpr int G = kOrthoThreads / NT;
     static constexpr int R = SP <= 20 ? 128 : 64;  // rows per slab
-    static constexpr int V4 = R * SP / 4;          // float4 per slab and operand
-    static constexpr int PF = (V4 + 255) / 256;    // float4 per thread and operand
-    static constexpr int kStage = 2 * R * SP;      // doubles
-    static constexpr int kReduce = G * NT * 9;     // doubles
-    static constexpr int kSmem = kStage > kReduce ? kStage : kReduce;
-    static_assert(kSmem * 8 <= 48 * 1024, "static shared memory");
+    static constexpr int kRounds = (R + G - 1) / G;  // rows of a group in a slab
+    static constexpr int kStage = kRounds * G;     // rows staged at a time
+    static constexpr int kTile = NT * 9;           // doubles of a group's tiles
 };
 
 template <int S, int SP>
-__global__ void __launch_bounds__(256)
-    gram_kernel(const Chunk* __restrict__ chunks, const float* __restrict__ A,
-                const float* __restrict__ B, double* __restrict__ G) {
+struct GramTile {
     using Sh = GramShape<S, SP>;
-    __shared__ double sm[Sh::kSmem];
-    // A^T A (every orthonormalisation) stages one operand; A^T B (the Ritz
-    // step) two
-    const bool same = A == B;
-    double* As = sm;
-    double* Bs = same ? sm : sm + Sh::R * SP;
-    const Chunk ch = chunks[blockIdx.x];
-    const int tid = threadIdx.x;
-    const bool worker = tid < Sh::G * Sh::NT;
-    const int tile = tid % Sh::NT, grp = tid / Sh::NT;
-    int tp = 0, tq = tile;  // tile (tp, tq), tp <= tq
-    while (tq >= Sh::T - tp) {
-        tq -= Sh::T - tp;
-        ++tp;
-    }
-    tq += tp;
     double acc[3][3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) acc[i][j] = 0.0;
-
-    float4 pa[Sh::PF], pb[Sh::PF];
-    auto prefetch = [&](int r0) {
-        const int rows = min(Sh::R, ch.end - r0);
-        const float4* a4 = reinterpret_cast<const float4*>(A + static_cast<int64_t>(r0) * SP);
-        const float4* b4 = reinterpret_cast<const float4*>(B + static_cast<int64_t>(r0) * SP);
-#pragma unroll
-        for (int k = 0; k < Sh::PF; ++k) {
-            const int e = tid + k * 256;
-            if (e < rows * SP / 4) {
-                pa[k] = a4[e];
-                if (!same) pb[k] = b4[e];
-            }
-        }
-    };
-    if (ch.start < ch.end) prefetch(ch.start);
-    for (int r0 = ch.start; r0 < ch.end; r0 += Sh::R) {
-        const int rows = min(Sh::R, ch.end - r0);
-        __syncthreads();  // the previous slab's products are done
-#pragma unroll
-        for (int k = 0; k < Sh::PF; ++k) {
-            const int e = tid + k * 256;
-            if (e < rows * SP / 4) {
-                As[4 * e] = pa[k].x;
-                As[4 * e + 1] = pa[k].y;
-                As[4 * e + 2] = pa[k].z;
-                As[4 * e + 3] = pa[k].w;
-                if (!same) {
-                    Bs[4 * e] = pb[k].x;
-                    Bs[4 * e + 1] = pb[k].y;
-                    Bs[4 * e + 2] = pb[k].z;
-                    Bs[4 * e + 3] = pb[k].w;
-                }
-            }
-        }
-        __syncthreads();
-        if (r0 + Sh::R < ch.end) prefetch(r0 + Sh::R);
-        if (worker) {
-            for (int r = grp; r < rows; r += Sh::G) {
-                const double* ar = As + r * SP + 3 * tp;
-                const double* br = Bs + r * SP + 3 * tq;
-                const double a0 = ar[0], a1 = ar[1], a2 = ar[2];
-                const double b0 = br[0], b1 = br[1], b2 = br[2];
-                acc[0][0] = fma(a0, b0, acc[0][0]);
-                acc[0][1] = fma(a0, b1, acc[0][1]);
-                acc[0][2] = fma(a0, b2, acc[0][2]);
-                acc[1][0] = fma(a1, b0, acc[1][0]);
-                acc[1][1] = fma(a1, b1, acc[1][1]);
-                acc[1][2] = fma(a1, b2, acc[1][2]);
-                acc[2][0] = fma(a2, b0, acc[2][0]);
-                acc[2][1] = fma(a2, b1, acc[2][1]);
-                acc[2][2] = fma(a2, b2, acc[2][2]);
-            }
-        }
-    }
-    __syncthreads();  // the staging buffer becomes the reduction buffer
-    if (worker) {
+    int tile, grp, tp, tq;
+    bool worker;
+    __device__ __forceinline__ void init(int groups) {
+        const int tid = threadIdx.x;
+        worker = tid < groups * Sh::NT;
+        tile = tid % Sh::NT;
+        grp = tid / Sh::NT;
+        tile_at(tile, &tp, &tq);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) sm[(grp * Sh::NT + tile) * 9 + i * 3 + j] = acc[i][j];
+            for (int j = 0; j < 3; ++j) acc[i][j] = 0.0;
     }
-    __syncthreads();
-    for (int o = tid; o < Sh::NT * 9; o += 256) {
-        const int t = o / 9, ij = o - t * 9, i = ij / 3, j = ij - i * 3;
-        int p = 0, q = t;
-        while (q >= Sh::T - p) {
-            q -= Sh::T - p;
-            ++p;
+    // tile t covers rows 3 p.., columns 3 q.., p <= q
+    static __device__ __forceinline__ void tile_at(int t, int* p, int* q) {
+        int pp = 0, qq = t;
+        while (qq >= Sh::T - pp) {
+            qq -= Sh::T - pp;
+            ++pp;
         }
-        q += p;
-        const int ea = 3 * p + i, eb = 3 * q + j;
-        if (ea > eb) continue;  // lower part of a diagonal tile
-        double v = 0.0;
-        for (int g = 0; g < Sh::G; ++g) v += sm[(g * Sh::NT + t) * 9 + ij];
-        atomicAdd(&G[static_cast<int64_t>(ch.slot) * S * S + ea * S + eb], v);
+        *p = pp;
+        *q = qq + pp;
     }
-}
+    __device__ __forceinline__ void add(const double* As, const double* Bs, int rows, int groups) {
+        if (!worker) return;
+#pragma unroll 2
+        for (int r = grp; r < rows; r += groups) {
+            const double* ar = As + r * SP + 3 * tp;
+            const double* br = Bs + r * SP + 3 * tq;
+            const double a0 = ar[0], a1 = ar[1], a2 = ar[2];
+            const double b0 = br[0], b1 = br[1], b2 = br[2];
+            acc[0][0] = fma(a0, b0, acc[0][0]);
+            acc[0][1] = fma(a0, b1, acc[0][1]);
+            acc[0][2] = fma(a0, b2, acc[0][2]);
+            acc[1][0] = fma(a1, b0, acc[1][0]);
+            acc[1][1] = fma(a1, b1, acc[1][1]);
+            acc[1][2] = fma(a1, b2, acc[1][2]);
+            acc[2][0] = fma(a2, b0, acc[2][0]);
+            acc[2][1] = fma(a2, b1, acc[2][1]);
+            acc[2][2] = fma(a2, b2, acc[2][2]);
+        }
+    }
+    __device__ __forceinline__ void store(double* to) const {
+        if (!worker) return;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) to[grp * Sh::kTile + tile * 9 + i * 3 + j] = acc[i][j];
+    }
+    // entry o of a group's tiles: row and column, false in the lower triangle
+    static __device__ __forceinline__ bool entry(int o, int* row, int* col) {
+        const int t = o / 9, ij = o - t * 9, i = ij / 3;
+        int p, q;
+        tile_at(t, &p, &q);
+        *row = 3 * p + i;
+        *col = 3 * q + ij - i * 3;
+        return *row <= *col;
+    }
+};
 
-// G = L L^T per slot, one warp: lane i keeps row i; right-looking updates
+// G = L L^T of one slot, one warp: lane i keeps row i; right-looking updates
 // with the pivot column shared by shuffles.  A pivot <= 1e-12 is the MGS
-// failure of the reference (column norm^2 after projection).
+// failure of the reference (column norm^2 after projection); the factor is
+// then the identity.  `g` (shared memory) holds the upper triangle.
 template <int S>
-__global__ void chol_kernel(const double* __restrict__ G, double* __restrict__ Lout,
-                            double* __restrict__ dinv, int* __restrict__ fail) {
-    const int slot = blockIdx.x;
-    const int lane = threadIdx.x;
-    const double* g = G + static_cast<int64_t>(slot) * S * S;
+__device__ void chol_factor(const double* g, double* Lout, double* dinv, int* fail) {
+    const int lane = threadIdx.x & 31;
     double row[S];
 #pragma unroll
     for (int k = 0; k < S; ++k) {
@@ -487,6 +445,7 @@ __global__ void chol_kernel(const double* __restrict__ G, double* __restrict__ L
         row[k] = v;
     }
     bool ok = true;
+    double diag = 1.0;
 #pragma unroll
     for (int j = 0; j < S; ++j) {
         const double pivot = __shfl_sync(0xffffffffu, row[j], j);
@@ -496,105 +455,278 @@ __global__ void chol_kernel(const double* __restrict__ G, double* __restrict__ L
         }
         const double ljj = sqrt(pivot);
         const double lij = lane == j ? ljj : row[j] / ljj;
+        if (lane == j) diag = ljj;
         if (lane >= j) row[j] = lij;
 #pragma unroll
         for (int k = j + 1; k < S; ++k) {
             const double lkj = __shfl_sync(0xffffffffu, lij, k);
-            if (lane > j) row[k] -= lij * lkj;
+            if (lane > j) row[k] = fma(-lij, lkj, row[k]);
         }
     }
-    if (!ok) {
-        if (lane == 0) fail[slot] = 1;
-        if (lane < S) {
-#pragma unroll
-            for (int k = 0; k < S; ++k) Lout[static_cast<int64_t>(slot) * S * S + lane * S + k] = lane == k;
-            dinv[slot * S + lane] = 1.0;
-        }
-        return;
-    }
+    if (!ok && lane == 0) *fail = 1;
     if (lane < S) {
 #pragma unroll
-        for (int k = 0; k < S; ++k)
-            Lout[static_cast<int64_t>(slot) * S * S + lane * S + k] = k <= lane ? row[k] : 0.0;
-        dinv[slot * S + lane] = 1.0 / row[lane];
+        for (int k = 0; k < S; ++k)  // column-major: the solve reads columns
+            Lout[k * S + lane] = ok ? (k <= lane ? row[k] : 0.0) : (k == lane ? 1.0 : 0.0);
+        dinv[lane] = ok ? 1.0 / diag : 1.0;
     }
 }
 
-// X = Y L^-T by forward substitution per row, FP64.  A block takes 256
-// consecutive rows: they are staged in shared memory with coalesced loads,
-// solved in place, and written back with coalesced stores (a row stride of
-// SP floats, a multiple of 4, keeps the 16-byte shared accesses of a
-// quarter-warp on distinct banks).  Each thread solves rows t and t + 128;
-// when both lie in the same slot (the common case: slots are contiguous
-// position ranges of at least 128 rows) every load of L serves both rows.
-constexpr int kApplyRows = 256;
-constexpr int kApplyThreads = 128;
+struct OrthoArgs {
+    const Chunk* chunks;
+    const float* Y;
+    float* X;
+    double* L;       // [slot][S][S], column-major
+    double* dinv;    // [slot][S]: 1 / diagonal
+    double* part;    // [chunk][G][kTile]: tiles of the groups, where a chunk has several CTAs
+    double* sums;    // [chunk][kTile]: Gram matrices of the chunks
+    double* bundle;  // [bundle][kTile]: sums of kBundle chunks each
+    int* chunk_done;   // CTAs done with the chunk; 0 between launches
+    int* bundle_done;  // chunks done of the bundle; 0 between launches
+    int* slot_done;    // bundles done of the slot; 0 between launches
+    int* fail;
+    int groups;      // row groups of a CTA (blockIdx.y takes the next `groups`)
+};
 
-template <int S, int SP, int NR>
-__device__ __forceinline__ void solve_rows(float* const (&row)[NR], const double* __restrict__ Ls,
-                                           const double* __restrict__ di) {
-    double x[NR][S];
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-        double v[NR];
-#pragma unroll
-        for (int q = 0; q < NR; ++q) v[q] = static_cast<double>(row[q][c]);
-#pragma unroll
-        for (int a = 0; a < c; ++a) {
-            const double l = __ldg(Ls + c * S + a);
-#pragma unroll
-            for (int q = 0; q < NR; ++q) v[q] -= x[q][a] * l;
-        }
-        const double d = __ldg(di + c);
-#pragma unroll
-        for (int q = 0; q < NR; ++q) x[q][c] = v[q] * d;
+// One pass of CholQR2, which is gram | solve + gram | solve:
+//   kSolve: X = Y L^-T by forward substitution, FP64 (else X is Y);
+//   kGram:  the Gram matrix of X; the last CTA of a slot factors it.
+// A chunk's row groups are dealt to several CTAs where there are few chunks;
+// each solves and sums only the rows of its groups, and the sums are added in
+// the same order however they are dealt (groups in order, then chunks in
+// order, kBundle at a time), so the factor does not depend on the split or on
+// timing.
+//
+// Bound by the FP64 operands' way through shared memory at 1M rows and by
+// latency at 20,000 and fewer: the launch, the slabs of one CTA, and the
+// factor's chain of 18 square roots and divisions.  An orthonormalisation (two
+// passes) of 18 columns takes 34 us of kernels in 3 launches at 1,000 rows, 41
+// at 20,000 and 255 at 1M; as eight launches (clear, Gram matrix, factor and
+// solve, twice, with a chunk on one CTA) it took 56, 61 and 268.  Splitting a
+// chunk is what shortens it at few rows (a CTA walks 88 to 176 rows, not 1024);
+// from 149 chunks on every SM has one and the whole chunk stays on one CTA, with
+// no tiles through global memory (with the split's row arithmetic the 1M rows
+// took 354 us).
+template <int S, int SP, bool kSolve, bool kGram, bool kSplit>
+__global__ void __launch_bounds__(kOrthoThreads, 2) ortho_kernel(const OrthoArgs p) {
+    using Sh = GramShape<S, SP>;
+    constexpr int kVec = SP / 4;
+    constexpr int kPf = (Sh::kStage * kVec + kOrthoThreads - 1) / kOrthoThreads;
+    constexpr int kReduce = (Sh::G + 1) * Sh::kTile;  // the groups' tiles and their sum
+    constexpr int kDoubles = Sh::kStage * SP > kReduce ? Sh::kStage * SP : kReduce;
+    static_assert(Sh::kStage <= kOrthoThreads, "a thread solves one row");
+    __shared__ __align__(16) float rows_f[kSolve ? Sh::kStage * SP : 4];
+    __shared__ __align__(16) double Ls[S * S];
+    __shared__ double di[S];
+    __shared__ __align__(16) double sm[kGram ? kDoubles : 2];
+    __shared__ bool last;
+    const Chunk ch = p.chunks[blockIdx.x];
+    const int tid = threadIdx.x;
+    const int rows = ch.end - ch.start;
+    // Staged rows are whole rounds of the CTA's groups; where a chunk is split,
+    // the last round of a slab may run past the slab and is padded with zeros,
+    // which change no sum.
+    int g0 = 0, groups = Sh::G, local = rows, stage = Sh::R, per_slab = Sh::R;
+    if (kSplit) {
+        g0 = blockIdx.y * p.groups;
+        groups = min(p.groups, Sh::G - g0);
+        per_slab = Sh::kRounds * groups;
+        local = (rows + Sh::R - 1) / Sh::R * per_slab;
+        stage = Sh::kStage / groups * groups;
     }
+    // staged row j -> row of the chunk; false for padding
+    auto row_of = [&](int j, int* row) {
+        *row = j;
+        if (!kSplit) return true;
+        const int slab = j / per_slab, in = j - slab * per_slab, round = in / groups;
+        const int r = round * Sh::G + g0 + in - round * groups;
+        *row = slab * Sh::R + r;
+        return r < Sh::R && *row < rows;
+    };
+    float4 pf[kPf];
+    const float4* y4 = reinterpret_cast<const float4*>(p.Y + static_cast<int64_t>(ch.start) * SP);
+    float4* x4 = reinterpret_cast<float4*>(p.X + static_cast<int64_t>(ch.start) * SP);
+    auto prefetch = [&](int j0) {
 #pragma unroll
-    for (int q = 0; q < NR; ++q) {
-        float4* r4 = reinterpret_cast<float4*>(row[q]);
-#pragma unroll
-        for (int v = 0; v < SP / 4; ++v) {
-            float o[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                o[k] = 4 * v + k < S ? static_cast<float>(x[q][4 * v + k]) : 0.0f;
-            r4[v] = make_float4(o[0], o[1], o[2], o[3]);
+        for (int k = 0; k < kPf; ++k) {
+            const int e = tid + k * kOrthoThreads, j = e / kVec;
+            int row;
+            pf[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (j < stage && j0 + j < local && row_of(j0 + j, &row))
+                pf[k] = y4[static_cast<int64_t>(row) * kVec + e - j * kVec];
         }
+    };
+    prefetch(0);
+    if (kSolve) {
+        for (int e = tid; e < S * S; e += kOrthoThreads)
+            Ls[e] = __ldcg(p.L + static_cast<int64_t>(ch.slot) * S * S + e);
+        if (tid < S) di[tid] = __ldcg(p.dinv + static_cast<int64_t>(ch.slot) * S + tid);
     }
-}
-
-template <int S, int SP>
-__global__ void __launch_bounds__(kApplyThreads)
-    apply_kernel(int64_t cnt, const int32_t* __restrict__ slot_of_pos,
-                 const double* __restrict__ L, const double* __restrict__ dinv,
-                 const float* __restrict__ Y, float* __restrict__ X) {
-    __shared__ __align__(16) float rows[kApplyRows * SP];
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * kApplyRows;
-    const int nrows = static_cast<int>(min(static_cast<int64_t>(kApplyRows), cnt - r0));
-    const float4* y4 = reinterpret_cast<const float4*>(Y + r0 * SP);
-    float4* s4 = reinterpret_cast<float4*>(rows);
-    for (int e = threadIdx.x; e < nrows * SP / 4; e += kApplyThreads) s4[e] = y4[e];
-    __syncthreads();
-    const int ta = threadIdx.x, tb = threadIdx.x + kApplyThreads;
-    const int sa = ta < nrows ? slot_of_pos[r0 + ta] : -1;
-    const int sb = tb < nrows ? slot_of_pos[r0 + tb] : -1;
-    auto Lof = [&](int slot) { return L + static_cast<int64_t>(slot) * S * S; };
-    if (sa >= 0 && sa == sb) {
-        float* const both[2] = {rows + ta * SP, rows + tb * SP};
-        solve_rows<S, SP, 2>(both, Lof(sa), dinv + sa * S);
+    auto widen = [&](int e, const float4& q) {
+        reinterpret_cast<double2*>(sm)[2 * e] =
+            make_double2(static_cast<double>(q.x), static_cast<double>(q.y));
+        reinterpret_cast<double2*>(sm)[2 * e + 1] =
+            make_double2(static_cast<double>(q.z), static_cast<double>(q.w));
+    };
+    GramTile<S, SP> gt;
+    if (kGram) gt.init(groups);
+    for (int j0 = 0; j0 < local; j0 += stage) {
+        const int n = min(stage, local - j0);
+        __syncthreads();  // the previous stage is done with
+#pragma unroll
+        for (int k = 0; k < kPf; ++k) {
+            const int e = tid + k * kOrthoThreads;
+            if (e >= n * kVec) break;
+            if (kSolve) {
+                reinterpret_cast<float4*>(rows_f)[e] = pf[k];
+            } else {
+                widen(e, pf[k]);
+            }
+        }
+        __syncthreads();
+        if (j0 + stage < local) prefetch(j0 + stage);
+        if (kSolve) {
+            if (tid < n) {
+                float4* r4 = reinterpret_cast<float4*>(rows_f) + tid * kVec;
+                double v[SP];
+#pragma unroll
+                for (int q = 0; q < kVec; ++q) {
+                    const float4 y = r4[q];
+                    v[4 * q] = static_cast<double>(y.x);
+                    v[4 * q + 1] = static_cast<double>(y.y);
+                    v[4 * q + 2] = static_cast<double>(y.z);
+                    v[4 * q + 3] = static_cast<double>(y.w);
+                }
+                // column by column: every entry still gets its terms in order
+#pragma unroll
+                for (int a = 0; a < S; ++a) {
+                    v[a] *= di[a];
+#pragma unroll
+                    for (int c = a & ~1; c < S; c += 2) {
+                        if (c + 1 <= a) continue;
+                        const double2 l = *reinterpret_cast<const double2*>(Ls + a * S + c);
+                        if (c > a) v[c] = fma(-v[a], l.x, v[c]);
+                        v[c + 1] = fma(-v[a], l.y, v[c + 1]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < kVec; ++q) {
+                    float o[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        o[k] = 4 * q + k < S ? static_cast<float>(v[4 * q + k]) : 0.0f;
+                    r4[q] = make_float4(o[0], o[1], o[2], o[3]);
+                }
+            }
+            __syncthreads();
+            for (int e = tid; e < n * kVec; e += kOrthoThreads) {
+                const int j = e / kVec;
+                const float4 x = reinterpret_cast<const float4*>(rows_f)[e];
+                int row;
+                if (row_of(j0 + j, &row)) x4[static_cast<int64_t>(row) * kVec + e - j * kVec] = x;
+                if (kGram) widen(e, x);
+            }
+            if (kGram) __syncthreads();
+        }
+        if (kGram) gt.add(sm, sm, n, groups);
+    }
+    if (!kGram) return;
+    // true in the last of `of` CTAs to get here; its reads then see their writes
+    auto last_of = [&](int* counter, int of) {
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            last = atomicAdd(counter, 1) == of - 1;
+            if (last) *counter = 0;
+        }
+        __syncthreads();
+        __threadfence();
+        return last;
+    };
+    // `to` = the sum of `of` tile sets from `from`, in order
+    auto sum = [&](const double* from, int of, double* to) {
+        for (int o = tid; o < Sh::kTile; o += kOrthoThreads) {
+            double v = 0.0;
+#pragma unroll 16
+            for (int k = 0; k < of; ++k) v += __ldcg(from + static_cast<int64_t>(k) * Sh::kTile + o);
+            to[o] = v;
+        }
+    };
+    // the chunk's matrix: its groups in order
+    const int64_t chunk = blockIdx.x;
+    const int bundles = (ch.of + kBundle - 1) / kBundle;
+    const int in_slot = static_cast<int>(chunk) - ch.first, bundle = in_slot / kBundle;
+    double* const mat = sm + (kSplit ? 0 : Sh::G * Sh::kTile);
+    double* to = ch.of == 1 ? mat : p.sums + chunk * Sh::kTile;
+    if (kSplit) {
+        double* part = p.part + chunk * Sh::G * Sh::kTile;
+        gt.store(part + static_cast<int64_t>(g0) * Sh::kTile);
+        if (!last_of(p.chunk_done + chunk, gridDim.y)) return;
+        sum(part, Sh::G, to);
     } else {
-        if (sa >= 0) {
-            float* const one[1] = {rows + ta * SP};
-            solve_rows<S, SP, 1>(one, Lof(sa), dinv + sa * S);
+        __syncthreads();  // the staging buffer becomes the reduction buffer
+        gt.store(sm);
+        __syncthreads();
+        for (int o = tid; o < Sh::kTile; o += kOrthoThreads) {
+            double v = 0.0;
+#pragma unroll
+            for (int g = 0; g < Sh::G; ++g) v += sm[g * Sh::kTile + o];
+            to[o] = v;
         }
-        if (sb >= 0) {
-            float* const one[1] = {rows + tb * SP};
-            solve_rows<S, SP, 1>(one, Lof(sb), dinv + sb * S);
+    }
+    if (ch.of > 1) {  // its bundle's chunks in order, then the slot's bundles
+        if (!last_of(p.bundle_done + ch.bundle + bundle, min(kBundle, ch.of - bundle * kBundle))) return;
+        to = bundles == 1 ? mat : p.bundle + static_cast<int64_t>(ch.bundle + bundle) * Sh::kTile;
+        sum(p.sums + static_cast<int64_t>(ch.first + bundle * kBundle) * Sh::kTile,
+            min(kBundle, ch.of - bundle * kBundle), to);
+        if (bundles > 1) {
+            if (!last_of(p.slot_done + ch.slot, bundles)) return;
+            sum(p.bundle + static_cast<int64_t>(ch.bundle) * Sh::kTile, bundles, mat);
         }
     }
     __syncthreads();
-    float4* x4 = reinterpret_cast<float4*>(X + r0 * SP);
-    for (int e = threadIdx.x; e < nrows * SP / 4; e += kApplyThreads) x4[e] = s4[e];
+    for (int o = tid; o < Sh::kTile; o += kOrthoThreads) {
+        int row, col;
+        if (GramTile<S, SP>::entry(o, &row, &col)) Ls[row * S + col] = mat[o];
+    }
+    __syncthreads();
+    if (tid < 32)
+        chol_factor<S>(Ls, p.L + static_cast<int64_t>(ch.slot) * S * S,
+                       p.dinv + static_cast<int64_t>(ch.slot) * S, p.fail + ch.slot);
+}
+
+// A^T B of every slot (the Ritz step, once a run), added to a cleared G.
+template <int S, int SP>
+__global__ void __launch_bounds__(kOrthoThreads)
+    ritz_gram_kernel(const Chunk* __restrict__ chunks, const float* __restrict__ A,
+                     const float* __restrict__ B, double* __restrict__ G) {
+    using Sh = GramShape<S, SP>;
+    constexpr int kDoubles = 2 * Sh::R * SP > Sh::G * Sh::kTile ? 2 * Sh::R * SP : Sh::G * Sh::kTile;
+    static_assert(kDoubles * 8 <= 48 * 1024, "static shared memory");
+    __shared__ double sm[kDoubles];
+    const Chunk ch = chunks[blockIdx.x];
+    GramTile<S, SP> gt;
+    gt.init(Sh::G);
+    for (int r0 = ch.start; r0 < ch.end; r0 += Sh::R) {
+        const int rows = min(Sh::R, ch.end - r0);
+        __syncthreads();  // the previous slab is done with
+        for (int e = threadIdx.x; e < rows * SP; e += kOrthoThreads) {
+            sm[e] = static_cast<double>(A[static_cast<int64_t>(r0) * SP + e]);
+            sm[Sh::R * SP + e] = static_cast<double>(B[static_cast<int64_t>(r0) * SP + e]);
+        }
+        __syncthreads();
+        gt.add(sm, sm + Sh::R * SP, rows, Sh::G);
+    }
+    __syncthreads();
+    gt.store(sm);
+    __syncthreads();
+    for (int o = threadIdx.x; o < Sh::kTile; o += kOrthoThreads) {
+        int row, col;
+        if (!GramTile<S, SP>::entry(o, &row, &col)) continue;
+        double v = 0.0;
+        for (int g = 0; g < Sh::G; ++g) v += sm[g * Sh::kTile + o];
+        atomicAdd(&G[static_cast<int64_t>(ch.slot) * S * S + row * S + col], v);
+    }
 }
 
 // coords = X V (V: s x dim per slot), FP64; and per-slot max |coord|.
@@ -823,6 +955,7 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
     const int64_t m = g.n_edges;
     const int64_t n_slots = static_cast<int64_t>(it_comps.size());
     std::vector<int32_t> nodes_h, slot_h;
+    std::vector<int32_t> slot_end;
     std::vector<Chunk> chunks;
     std::vector<uint64_t> slot_seed(n_slots), noise_seed(n_slots);
     std::vector<float> expand_target(n_slots), slot_anchor(n_slots * dim);
@@ -834,8 +967,7 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
             slot_h.push_back(static_cast<int32_t>(sl));
         }
         const int32_t end = static_cast<int32_t>(nodes_h.size());
-        for (int32_t st = base; st < end; st += 1024)
-            chunks.push_back({static_cast<int32_t>(sl), st, std::min(end, st + 1024)});
+        slot_end.push_back(end);
         slot_seed[sl] = cseed[c];
         noise_seed[sl] = multi ? seed ^ (static_cast<uint64_t>(c + 1) * 0x94D049BBULL)
                                : seed ^ 0x5DEECE66DULL;
@@ -843,6 +975,21 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
         for (int k = 0; k < dim; ++k) slot_anchor[sl * dim + k] = multi ? anchors[c * dim + k] : 0.0f;
     }
     const int64_t cnt = static_cast<int64_t>(nodes_h.size());
+    // Chunks of 1024 rows, of more where that would make over two an SM (a
+    // slot's last CTA adds its chunks' matrices one after the other).
+    constexpr int64_t kOrthoCtas = 2 * 148;
+    int32_t n_bundles = 0;
+    const int32_t per_chunk =
+        static_cast<int32_t>(std::max<int64_t>(1024, ceil_div(ceil_div(cnt, kOrthoCtas), 128) * 128));
+    for (int64_t sl = 0; sl < n_slots; ++sl) {
+        const int32_t base = sl ? slot_end[sl - 1] : 0, end = slot_end[sl];
+        const int32_t of = static_cast<int32_t>(ceil_div(end - base, per_chunk));
+        const int32_t first = static_cast<int32_t>(chunks.size());
+        for (int32_t st = base; st < end; st += per_chunk)
+            chunks.push_back({static_cast<int32_t>(sl), st, std::min(end, st + per_chunk), first, of,
+                              n_bundles});
+        n_bundles += static_cast<int32_t>(ceil_div(of, kBundle));
+    }
     DevBuf<int32_t> nodes(cnt, s), slots(cnt, s), pos(n, s), plen(cnt, s), quads(cnt + 1, s),
         qptr(cnt + 1, s), long_rows(cnt, s), n_long(1, s);
     DevBuf<Chunk> dch(chunks.size(), s);
@@ -892,29 +1039,41 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
     UMAPB_LAUNCH_CHECK();
 
     DevBuf<float> Xb(cnt * SP, s), Yb(cnt * SP, s);
-    DevBuf<double> G(n_slots * S * S, s), L(n_slots * S * S, s), dg(n_slots * S, s);
-    DevBuf<int> fail(n_slots, s);
+    using Sh = GramShape<S, SP>;
+    const unsigned nch = static_cast<unsigned>(chunks.size());
+    const unsigned gr = grid_for(cnt);
+    // few chunks: a chunk's row groups on as many CTAs as keep two an SM
+    const int split = static_cast<int>(
+        std::max<int64_t>(1, std::min<int64_t>(Sh::G, kOrthoCtas / static_cast<int64_t>(nch))));
+    const int groups = static_cast<int>(ceil_div(Sh::G, split));
+    const dim3 ortho_grid(nch, static_cast<unsigned>(ceil_div(Sh::G, groups)));
+    DevBuf<double> G(n_slots * S * S, s), L(n_slots * S * S, s), dinv(n_slots * S, s),
+        sums(static_cast<int64_t>(nch) * Sh::kTile, s),
+        bundle_sums(static_cast<int64_t>(n_bundles) * Sh::kTile, s),
+        part(ortho_grid.y > 1 ? static_cast<int64_t>(nch) * Sh::G * Sh::kTile : 1, s);
+    DevBuf<int> fail(n_slots, s), chunk_done(nch, s), bundle_done(n_bundles, s), slot_done(n_slots, s);
     UMAPB_CUDA(cudaMemsetAsync(fail.get(), 0, n_slots * 4, s));
+    UMAPB_CUDA(cudaMemsetAsync(chunk_done.get(), 0, nch * 4, s));
+    UMAPB_CUDA(cudaMemsetAsync(bundle_done.get(), 0, n_bundles * 4, s));
+    UMAPB_CUDA(cudaMemsetAsync(slot_done.get(), 0, n_slots * 4, s));
     init_block_kernel<<<grid_for(cnt), 256, 0, s>>>(nodes.get(), cnt, slots.get(), dseed.get(),
                                                     deg.get(), S, SP, Xb.get());
     UMAPB_LAUNCH_CHECK();
-    const unsigned nch = static_cast<unsigned>(chunks.size());
-    const unsigned gr = grid_for(cnt);
-    const unsigned ga = grid_for(cnt, kApplyRows);
     // CholQR2: src -> dst -> src; the orthonormal block ends in src
     auto cholqr = [&](float* src, float* dst) {
-        for (int pass = 0; pass < 2; ++pass) {
-            float* a = pass == 0 ? src : dst;
-            float* b = pass == 0 ? dst : src;
-            UMAPB_CUDA(cudaMemsetAsync(G.get(), 0, n_slots * S * S * 8, s));
-            gram_kernel<S, SP><<<nch, 256, 0, s>>>(dch.get(), a, a, G.get());
+        OrthoArgs oa{dch.get(),          src,        nullptr,           L.get(),
+                     dinv.get(),         part.get(), sums.get(),        bundle_sums.get(),
+                     chunk_done.get(),   bundle_done.get(), slot_done.get(), fail.get(), groups};
+        auto pass = [&](auto kernel, auto split_kernel, const float* y, float* x) {
+            oa.Y = y;
+            oa.X = x;
+            (ortho_grid.y > 1 ? split_kernel : kernel)<<<ortho_grid, kOrthoThreads, 0, s>>>(oa);
             UMAPB_LAUNCH_CHECK();
-            chol_kernel<S><<<static_cast<unsigned>(n_slots), 32, 0, s>>>(G.get(), L.get(), dg.get(),
-                                                                        fail.get());
-            UMAPB_LAUNCH_CHECK();
-            apply_kernel<S, SP><<<ga, kApplyThreads, 0, s>>>(cnt, slots.get(), L.get(), dg.get(), a, b);
-            UMAPB_LAUNCH_CHECK();
-        }
+        };
+        pass(ortho_kernel<S, SP, false, true, false>, ortho_kernel<S, SP, false, true, true>, src,
+             nullptr);
+        pass(ortho_kernel<S, SP, true, true, false>, ortho_kernel<S, SP, true, true, true>, src, dst);
+        pass(ortho_kernel<S, SP, true, false, false>, ortho_kernel<S, SP, true, false, true>, dst, src);
     };
     const unsigned gr_spmm = static_cast<unsigned>(
         n_long_h + ceil_div(cnt, static_cast<int64_t>(spmm_rows_per_block<SP>())));
@@ -933,7 +1092,7 @@ bool run_iterative(const std::vector<int64_t>& it_comps, const std::vector<int64
     }
     spmm(Xb.get(), Yb.get());
     UMAPB_CUDA(cudaMemsetAsync(G.get(), 0, n_slots * S * S * 8, s));
-    gram_kernel<S, SP><<<nch, 256, 0, s>>>(dch.get(), Xb.get(), Yb.get(), G.get());
+    ritz_gram_kernel<S, SP><<<nch, kOrthoThreads, 0, s>>>(dch.get(), Xb.get(), Yb.get(), G.get());
     UMAPB_LAUNCH_CHECK();
     std::vector<double> G_h(n_slots * S * S);
     std::vector<int> fail_h(n_slots);
