@@ -29,6 +29,7 @@ using namespace umapb;
 namespace {
 
 thread_local std::string g_last_error;
+std::atomic<int64_t> g_models{0};  // alive
 
 constexpr const char* kVersion = "1.1.4+b200.1";
 constexpr float kSmoothKTolerance = 1e-5f;  // lib.rs:19
@@ -177,22 +178,54 @@ void validate_csr_host(const int64_t* indptr, const int64_t* indices, const floa
     if (n_cols <= 0) invalid("csr n_cols must be >= 1");
     if (!indptr || (indptr[n_rows] > 0 && (!indices || !data))) invalid("null csr array");
     if (indptr[0] != 0) invalid("csr indptr must start from 0");
-    for (int64_t row = 0; row < n_rows; ++row) {
-        if (indptr[row] > indptr[row + 1])
-            invalid("csr indptr must be non-decreasing, got indptr[" + std::to_string(row) +
-                    "]=" + std::to_string(indptr[row]) + " > indptr[" + std::to_string(row + 1) +
-                    "]=" + std::to_string(indptr[row + 1]));
-        for (int64_t e = indptr[row] + 1; e < indptr[row + 1]; ++e)
-            if (indices[e - 1] >= indices[e])
-                invalid("csr row " + std::to_string(row) + " indices must be strictly increasing");
-        for (int64_t e = indptr[row]; e < indptr[row + 1]; ++e)
-            if (indices[e] < 0 || indices[e] >= n_cols)
-                invalid("csr row " + std::to_string(row) + " has column index " +
-                        std::to_string(indices[e]) + " out of bounds for n_cols=" +
-                        std::to_string(n_cols));
+    // Entries [0, nnz) in ranges over threads, of whole rows; where one finds a
+    // fault, the rows are walked in order for the first of them.  The offsets
+    // come before anything that they index.
+    const int64_t nnz = indptr[n_rows];
+    bool ordered = true;
+    for (int64_t row = 0; row < n_rows; ++row) ordered &= indptr[row] <= indptr[row + 1];
+    // 2M entries take 3.1 ms in order on one thread and 1.4 on four, 400,000 take
+    // 0.63 and, on two, 0.39.
+    constexpr int64_t kEntriesPerThread = 250000;
+    const int threads = static_cast<int>(
+        std::min<int64_t>(host_threads(), 1 + nnz / kEntriesPerThread));
+    std::atomic<bool> good{ordered};
+    if (ordered && nnz > 0)
+        run_threads(threads, [&](int t) {
+            auto row_from = [&](int k) {
+                return k == threads ? n_rows
+                                    : std::lower_bound(indptr, indptr + n_rows, nnz / threads * k) -
+                                          indptr;
+            };
+            bool ok = true;
+            const int64_t end = row_from(t + 1);
+            for (int64_t row = t == 0 ? 0 : row_from(t); row < end && ok; ++row) {
+                int64_t before = -1;
+                for (int64_t e = indptr[row]; e < indptr[row + 1]; ++e) {
+                    ok &= (indices[e] > before) & (indices[e] < n_cols) & std::isfinite(data[e]);
+                    before = indices[e];
+                }
+            }
+            if (!ok) good = false;
+        });
+    if (!good) {
+        for (int64_t row = 0; row < n_rows; ++row) {
+            if (indptr[row] > indptr[row + 1])
+                invalid("csr indptr must be non-decreasing, got indptr[" + std::to_string(row) +
+                        "]=" + std::to_string(indptr[row]) + " > indptr[" + std::to_string(row + 1) +
+                        "]=" + std::to_string(indptr[row + 1]));
+            for (int64_t e = indptr[row] + 1; e < indptr[row + 1]; ++e)
+                if (indices[e - 1] >= indices[e])
+                    invalid("csr row " + std::to_string(row) + " indices must be strictly increasing");
+            for (int64_t e = indptr[row]; e < indptr[row + 1]; ++e)
+                if (indices[e] < 0 || indices[e] >= n_cols)
+                    invalid("csr row " + std::to_string(row) + " has column index " +
+                            std::to_string(indices[e]) + " out of bounds for n_cols=" +
+                            std::to_string(n_cols));
+        }
+        for (int64_t e = 0; e < indptr[n_rows]; ++e)
+            if (!std::isfinite(data[e])) invalid("csr data must be finite");
     }
-    for (int64_t e = 0; e < indptr[n_rows]; ++e)
-        if (!std::isfinite(data[e])) invalid("csr data must be finite");
     if (indptr[n_rows] > 0x7FFFFFFFll) invalid("csr input above 2^31 nonzeros is not supported");
 }
 
@@ -508,8 +541,7 @@ void fit_device(umapb_model* m, const float* Xd, int64_t n, int64_t d, bool copy
 
 void upload(DevBuf<float>& dst, const float* src, int64_t count, cudaStream_t s) {
     dst.alloc(count, s);
-    if (count > 0)
-        UMAPB_CUDA(cudaMemcpyAsync(dst.get(), src, count * 4, cudaMemcpyHostToDevice, s));
+    upload_host(dst.get(), src, count * 4, s);
 }
 
 void copy_embedding_out(umapb_model* m, float* out) {
@@ -992,13 +1024,14 @@ int32_t umapb_create(const umapb_params* params, umapb_model** out_model) {
         if (params->metric < 0 || params->metric > UMAPB_METRIC_BRAYCURTIS)
             invalid("unsupported metric");
         auto* m = new umapb_model();
+        g_models.fetch_add(1);
         m->p = *params;
         *out_model = m;
     });
 }
 
-void umapb_destroy(umapb_model* m) {
-    if (!m) return;
+namespace {
+void destroy_model(umapb_model* m) {
     {
         std::lock_guard<std::mutex> lk(m->mu);
         if (m->stream) {
@@ -1018,6 +1051,14 @@ void umapb_destroy(umapb_model* m) {
         }
     }
     delete m;
+    g_models.fetch_sub(1);
+}
+}  // namespace
+
+void umapb_destroy(umapb_model* m) {
+    if (!m) return;
+    destroy_model(m);
+    if (g_models.load() == 0) trim_host_staging();
 }
 
 int32_t umapb_fit(umapb_model* m, const float* data, int64_t n_rows, int64_t n_cols) {
@@ -1088,7 +1129,7 @@ int32_t umapb_fit_transform_csr_stateless(const umapb_params* params, const int6
     if (st != UMAPB_OK) return st;
     st = umapb_fit_transform_csr(m, indptr, indices, data, n_rows, n_cols, out);
     const std::string err = g_last_error;
-    umapb_destroy(m);
+    destroy_model(m);
     g_last_error = err;
     return st;
 }
@@ -1130,7 +1171,7 @@ int32_t umapb_fit_transform_stateless(const umapb_params* params, const float* d
     if (st != UMAPB_OK) return st;
     st = umapb_fit_transform(m, data, n_rows, n_cols, out);
     const std::string err = g_last_error;
-    umapb_destroy(m);
+    destroy_model(m);
     g_last_error = err;
     return st;
 }
@@ -1377,10 +1418,6 @@ struct ScopedStream {
         }
     }
 };
-
-void to_i64(const std::vector<int32_t>& v, int64_t* out) {
-    for (size_t i = 0; i < v.size(); ++i) out[i] = v[i];
-}
 }  // namespace
 
 int32_t umapb_knn_exact(const float* data, int64_t n, int64_t d, int64_t k, int32_t metric,
@@ -1396,11 +1433,9 @@ int32_t umapb_knn_exact(const float* data, int64_t n, int64_t d, int64_t k, int3
         int64_t fb = 0;
         knn_exact_device(X.get(), n, X.get(), n, static_cast<int>(d), static_cast<int>(k), metric,
                          backend, idx.get(), dist.get(), &fb, nullptr, nullptr, ss.s);
-        std::vector<int32_t> ih(n * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_indices(indices, idx.get(), n * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, indices);
         if (fallback_rows) *fallback_rows = fb;
     });
 }
@@ -1420,11 +1455,9 @@ int32_t umapb_knn_query(const float* query, int64_t nq, const float* reference, 
         DevBuf<float> dist(nq * k, ss.s);
         knn_exact_device(Q.get(), nq, R.get(), nr, static_cast<int>(d), static_cast<int>(k),
                          metric, backend, idx.get(), dist.get(), nullptr, nullptr, nullptr, ss.s);
-        std::vector<int32_t> ih(nq * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), nq * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_indices(indices, idx.get(), nq * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), nq * k * 4, cudaMemcpyDeviceToHost, ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, indices);
     });
 }
 
@@ -1443,13 +1476,10 @@ int32_t umapb_knn_csr(const int64_t* indptr, const int64_t* indices, const float
         DevBuf<int32_t> idx(n_rows * k, ss.s);
         DevBuf<float> dist(n_rows * k, ss.s);
         knn_sparse(csr, csr, ci, true, static_cast<int>(k), metric, idx.get(), dist.get(), ss.s);
-        std::vector<int32_t> ih(n_rows * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_indices(out_idx, idx.get(), n_rows * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
                                    ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, out_idx);
     });
 }
 
@@ -1470,13 +1500,10 @@ int32_t umapb_nndescent_csr(const int64_t* indptr, const int64_t* indices, const
         NdStats st;
         const int64_t ran = nndescent_csr(csr, static_cast<int>(k), metric, candidate_pool,
                                           n_iters, seed, idx.get(), dist.get(), ss.s, &st);
-        std::vector<int32_t> ih(n_rows * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_indices(out_idx, idx.get(), n_rows * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
                                    ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, out_idx);
         if (iters_run) *iters_run = ran;
         if (candidates_evaluated) *candidates_evaluated = st.candidates;
         if (kernel_sec) *kernel_sec = st.kernel_sec;
@@ -1502,13 +1529,10 @@ int32_t umapb_knn_csr_query(const int64_t* q_indptr, const int64_t* q_indices,
         DevBuf<int32_t> idx(n_q * k, ss.s);
         DevBuf<float> dist(n_q * k, ss.s);
         knn_sparse(q, r, ri, false, static_cast<int>(k), metric, idx.get(), dist.get(), ss.s);
-        std::vector<int32_t> ih(n_q * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), n_q * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_indices(out_idx, idx.get(), n_q * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_q * k * 4, cudaMemcpyDeviceToHost,
                                    ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, out_idx);
     });
 }
 
@@ -1531,11 +1555,9 @@ int32_t umapb_nndescent(const float* data, int64_t n, int64_t d, int64_t k, int3
                                              dist.get(), ss.s, &st);
         if (candidates_evaluated) *candidates_evaluated = st.candidates;
         if (kernel_sec) *kernel_sec = st.kernel_sec;
-        std::vector<int32_t> ih(n * k);
-        UMAPB_CUDA(cudaMemcpyAsync(ih.data(), idx.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_indices(indices, idx.get(), n * k, ss.s);
         UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
-        to_i64(ih, indices);
         if (iters_run) *iters_run = ran;
     });
 }

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -70,6 +71,31 @@ struct CsrDevice {
     DevBuf<float> values;
     DevBuf<float> sq, l2;
 };
+
+// Host arrays (hostio.cu), copied in the order of `s` with cudaMemcpyAsync's
+// rules: pinned arrays are in use until `s` has been synchronised.
+int host_threads();
+void upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
+void download_indices(int64_t* dst, const int32_t* src, int64_t n, cudaStream_t s);
+void upload_indices(int32_t* dst, const int64_t* src, int64_t n, cudaStream_t s);
+// Frees the pinned buffers that no upload is using.
+void trim_host_staging();
+
+// work(0) .. work(threads - 1), work(0) on the calling thread, and all the
+// others too where no thread can be started.
+template <typename F>
+void run_threads(int threads, const F& work) {
+    std::vector<std::thread> team;
+    int t = 1;
+    try {
+        team.reserve(threads);
+        for (; t < threads; ++t) team.emplace_back(work, t);
+    } catch (const std::exception&) {
+    }
+    work(0);
+    for (; t < threads; ++t) work(t);
+    for (auto& th : team) th.join();
+}
 
 // Uploads host CSR arrays (already validated) and computes the norms.
 void csr_upload(const int64_t* indptr, const int64_t* indices, const float* values,

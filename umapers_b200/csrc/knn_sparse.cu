@@ -458,17 +458,11 @@ void csr_upload(const int64_t* indptr, const int64_t* indices, const float* valu
     out.n_cols = n_cols;
     out.nnz = nnz;
     out.indptr.alloc(n_rows + 1, s);
-    UMAPB_CUDA(cudaMemcpyAsync(out.indptr.get(), indptr, (n_rows + 1) * 8, cudaMemcpyHostToDevice,
-                               s));
-    std::vector<int32_t> idx32(static_cast<size_t>(nnz));
-    for (int64_t e = 0; e < nnz; ++e) idx32[e] = static_cast<int32_t>(indices[e]);
+    upload_host(out.indptr.get(), indptr, (n_rows + 1) * 8, s);
     out.indices.alloc(std::max<int64_t>(nnz, 1), s);
     out.values.alloc(std::max<int64_t>(nnz, 1), s);
-    if (nnz > 0) {
-        UMAPB_CUDA(cudaMemcpyAsync(out.indices.get(), idx32.data(), nnz * 4,
-                                   cudaMemcpyHostToDevice, s));
-        UMAPB_CUDA(cudaMemcpyAsync(out.values.get(), values, nnz * 4, cudaMemcpyHostToDevice, s));
-    }
+    upload_indices(out.indices.get(), indices, nnz, s);
+    upload_host(out.values.get(), values, nnz * 4, s);
     out.sq.alloc(std::max<int64_t>(n_rows, 1), s);
     out.l2.alloc(std::max<int64_t>(n_rows, 1), s);
     if (n_rows > 0) {
@@ -476,8 +470,7 @@ void csr_upload(const int64_t* indptr, const int64_t* indices, const float* valu
                                                             n_rows, out.sq.get(), out.l2.get());
         UMAPB_LAUNCH_CHECK();
     }
-    // the host copy of the indices must outlive the copy that reads it
-    UMAPB_CUDA(cudaStreamSynchronize(s));
+    UMAPB_CUDA(cudaStreamSynchronize(s));  // a caller's pinned arrays are read
 }
 
 void csr_from_dense(const float* X, int64_t n, int64_t d, CsrDevice& out, cudaStream_t s) {
