@@ -235,3 +235,33 @@ def test_chunked_host_transform_equals_device_path_and_gated_rows_are_row_local(
     np.testing.assert_array_equal(out_1[flags_1], out_h[:131_072][flags_1])
     # the network's rows are the same too (row-wise inference)
     np.testing.assert_array_equal(out_1[~flags_1], out_h[:131_072][~flags_1])
+
+
+# one tile a CTA and one row tile more than it; three tiles with a short last
+# CTA; just below and above four; a ragged last row tile each
+@pytest.mark.parametrize("rows", [302_976, 302_977, 455_041, 606_077, 606_209])
+def test_network_does_not_depend_on_the_tiles_per_cta(trained, rows):
+    """Rows pass through the network one by one, so a request equals the same
+    rows in pieces of 100,000, where every CTA has one tile."""
+    import torch
+
+    m, fit, query, _, _ = trained
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    q = torch.from_numpy(query).cuda()[torch.randint(0, query.shape[0], (rows,), generator=g,
+                                                     device="cuda")]
+    q += 0.5 * torch.randn(q.shape, generator=g, device="cuda")
+    lib = _lib.load()
+
+    def run(x):
+        out = torch.empty((x.shape[0], 2), device="cuda")
+        flags = torch.empty(x.shape[0], dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        _lib.check(lib.umapb_surrogate_transform_device(m._core._handle, x.data_ptr(), x.shape[0],
+                                                        x.shape[1], 0, out.data_ptr(),
+                                                        flags.data_ptr(), None))
+        return out, flags
+
+    out, flags = run(q)
+    for at in range(0, rows, 100_000):
+        o, f = run(q[at:at + 100_000].contiguous())
+        assert torch.equal(out[at:at + 100_000], o) and torch.equal(flags[at:at + 100_000], f)

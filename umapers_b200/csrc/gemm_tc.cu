@@ -1,18 +1,31 @@
 // gemm_tc.cu - BF16 tensor-core GEMM with fused epilogues, the building
 // block of the transform surrogate's forward and backward passes.
 //
-// C[M x N] = A[M x K] B[N x K]^T.  One CTA computes one 128 x 128 tile of C:
+// C[M x N] = A[M x K] B[N x K]^T.  A CTA computes one to four 128 x 128 tiles
+// of C, each with an accumulator of 128 TMEM columns:
 //   warp 0      TMA producer: k-blocks of A and B (64 bf16 columns each,
-//               SWIZZLE_128B) through a kStages-deep shared-memory ring;
-//   warp 1      allocates 128 TMEM columns; one thread issues
+//               SWIZZLE_128B) through a kStages-deep shared-memory ring that
+//               runs on from tile to tile;
+//   warp 1      allocates the TMEM columns; one thread issues
 //               tcgen05.mma kind::f16 (M = N = 128, K = 16) into them;
-//   warps 2..5  epilogue: each reads its 32 TMEM lanes (rows) with
-//               tcgen05.ld, 32 columns at a time, and applies the fused
-//               operation (bias + GELU, GELU backward, output head, row min).
+//   then one or two epilogue groups of four warps, each with its accumulator:
+//               a warp reads its 32 TMEM lanes (rows) with tcgen05.ld, 32
+//               columns at a time, and applies the fused operation (bias +
+//               GELU, GELU backward, output head, row min).
 // Tiles are numbered along N first, so the CTAs that share an A tile run
 // together and A is read from HBM once.  TMA loads read only this GPU's
 // memory and never multicast.  Every wait is bounded; a timeout sets a
 // device error word that gemm_take_error() reports.
+//
+// Bound by the epilogue's instructions (erff above all) on the wide shapes.
+// With one tile a CTA and one group, two CTAs an SM keep eight epilogue warps
+// there, and each waits for its own tile's loads and products first.  With two
+// groups the next tile is computed under the epilogue of this one, sixteen
+// epilogue warps an SM: 1M rows, 512 columns, K = 128 with GELU 1.05 -> 0.76
+// ms, K = 512 with GELU and head 1.28 -> 0.92, K = 128 with row minimum and
+// 256 columns 0.27 -> 0.15; a 1M-row inference 3.23 -> 2.49 ms.
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "tcgen05.cuh"
 
@@ -25,15 +38,26 @@ using namespace tc;
 
 constexpr int GM = 128, GN = 128;
 constexpr int kStages = 3;
+// Tiles of a CTA: one per kTilesPerStep tiles, at most four.  More tiles a CTA
+// keep it longer on its SM, which a kernel of another stream has to wait for
+// (the plain transform of gated rows beside the network): with four the 1M
+// rows above take 2.49 ms alone and 4.41 beside that transform, with eight
+// 2.39 and 4.54, on one persistent CTA an SM 2.24 and 4.60, with one tile 3.23
+// and 5.16.  Below about 300,000 rows of 512 columns that wait costs more than
+// the overlap gains (150,000 rows beside a transform: 1.67 ms with two tiles,
+// 1.63 with one), and with one tile the second group is left out.
+constexpr int64_t kTilesPerStep = 4736;  // 32 per SM
+constexpr int64_t kMaxTilesPerCta = 4;
 constexpr int kTileBytes = GM * kBK * 2;         // 16 KiB per operand k-block
 constexpr int kStageBytes = 2 * kTileBytes;      // A + B
 constexpr uint32_t kGemmIdesc = idesc_bf16(GM, GN);
-constexpr uint32_t kTmemCols = GN;
 
 struct GemmParams {
     int64_t M, N;
     int kb;           // K / 64
     int64_t n_tiles;  // column tiles
+    int64_t tiles;
+    int per_cta;      // tiles of a CTA
     GemmOut o;
 };
 
@@ -68,7 +92,7 @@ __device__ __forceinline__ void store_f32x32(float* dst, const float* v) {
 
 template <int EPI>
 __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, int64_t row,
-                                         int64_t n0, int64_t tile_n) {
+                                         int64_t n0, int64_t tile_n, uint32_t b_free) {
     const bool rv = row < p.M;
     const GemmOut& o = p.o;
     float head[kGemmMaxHead];
@@ -81,6 +105,11 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, in
         uint32_t r[32];
         tmem_ld32(taddr + 32 * c, r);
         tmem_wait_ld();
+        if (c == GN / 32 - 1) {  // the accumulator is read: the next tile may have it
+            fence_before();
+            __syncwarp();
+            if ((threadIdx.x & 31) == 0) mbar_arrive(b_free);
+        }
         const int64_t nb = n0 + 32 * c;
         float v[32];
 #pragma unroll
@@ -110,10 +139,16 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, in
 #pragma unroll
                 for (int h = 0; h < kGemmMaxHead; ++h) {
                     if (h < o.head_dim) {
-                        const float* w = o.head_w + h * p.N + nb;
+                        const float4* w4 = reinterpret_cast<const float4*>(o.head_w + h * p.N + nb);
                         float acc = 0.0f;
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) acc = fmaf(v[j], __ldg(w + j), acc);
+                        for (int q = 0; q < 8; ++q) {
+                            const float4 w = __ldg(w4 + q);
+                            acc = fmaf(v[4 * q], w.x, acc);
+                            acc = fmaf(v[4 * q + 1], w.y, acc);
+                            acc = fmaf(v[4 * q + 2], w.z, acc);
+                            acc = fmaf(v[4 * q + 3], w.w, acc);
+                        }
                         head[h] += acc;
                     }
                 }
@@ -160,8 +195,9 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, in
     }
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(192, 1)
+template <int EPI, int kGroups>
+// registers: two CTAs an SM of 192 threads or of 320
+__global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 GemmParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -172,29 +208,31 @@ __global__ void __launch_bounds__(192, 1)
     const uint32_t b_full = smem_u32(bars);
     const uint32_t b_empty = b_full + 8 * kStages;
     const uint32_t b_tfull = b_empty + 8 * kStages;
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 1);
+    const uint32_t b_tempty = b_tfull + 8 * kGroups;
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 2 * kGroups);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t tile = blockIdx.x;
-    const int64_t tile_n = tile % p.n_tiles;
-    const int64_t m0 = (tile / p.n_tiles) * GM;
-    const int64_t n0 = tile_n * GN;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(b_full + 8 * s, 1);
             mbar_init(b_empty + 8 * s, 1);
         }
-        mbar_init(b_tfull, 1);
+        for (int b = 0; b < kGroups; ++b) {
+            mbar_init(b_tfull + 8 * b, 1);
+            mbar_init(b_tempty + 8 * b, 4);  // one arrival per epilogue warp
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_holder), kTmemCols);
+    if (warp == 1) tmem_alloc(smem_u32(tmem_holder), kGroups * GN);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    const int64_t first = static_cast<int64_t>(blockIdx.x) * p.per_cta;
+    const int64_t end = min(first + p.per_cta, p.tiles);
 
     auto fail = [&](int code) {
         *abort_flag = 1;
@@ -203,49 +241,68 @@ __global__ void __launch_bounds__(192, 1)
 
     if (warp == 0) {
         if (lane == 0) {
-            for (int kb = 0; kb < p.kb; ++kb) {
-                const int st = kb % kStages;
-                const uint32_t round = static_cast<uint32_t>(kb / kStages);
-                if (!mbar_wait(b_empty + 8 * st, (round & 1) ^ 1, abort_flag)) {
-                    fail(1);
-                    break;
+            uint32_t step = 0;  // k-blocks so far
+            bool ok = true;
+            for (int64_t tile = first; ok && tile < end; ++tile) {
+                const int m0 = static_cast<int>(tile / p.n_tiles) * GM;
+                const int n0 = static_cast<int>(tile % p.n_tiles) * GN;
+                for (int kb = 0; kb < p.kb; ++kb, ++step) {
+                    const uint32_t st = step % kStages;
+                    if (!mbar_wait(b_empty + 8 * st, ((step / kStages) & 1) ^ 1, abort_flag)) {
+                        fail(1);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t sa = s0 + st * kStageBytes;
+                    mbar_expect_tx(b_full + 8 * st, kStageBytes);
+                    tma_load_2d(sa, &tmA, b_full + 8 * st, kb * kBK, m0);
+                    tma_load_2d(sa + kTileBytes, &tmB, b_full + 8 * st, kb * kBK, n0);
                 }
-                const uint32_t sa = s0 + st * kStageBytes;
-                mbar_expect_tx(b_full + 8 * st, kStageBytes);
-                tma_load_2d(sa, &tmA, b_full + 8 * st, kb * kBK, static_cast<int>(m0));
-                tma_load_2d(sa + kTileBytes, &tmB, b_full + 8 * st, kb * kBK, static_cast<int>(n0));
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
+            uint32_t step = 0, seq = 0;
             bool ok = true;
-            for (int kb = 0; kb < p.kb; ++kb) {
-                const int st = kb % kStages;
-                if (!mbar_wait(b_full + 8 * st, static_cast<uint32_t>((kb / kStages) & 1),
-                               abort_flag)) {
-                    fail(2);
-                    ok = false;
+            for (int64_t tile = first; ok && tile < end; ++tile, ++seq) {
+                const uint32_t buf = seq % kGroups;
+                if (!mbar_wait(b_tempty + 8 * buf, ((seq / kGroups) & 1) ^ 1, abort_flag)) {
+                    fail(4);
                     break;
                 }
                 fence_after();
-                const uint32_t sa = s0 + st * kStageBytes;
-                const uint64_t da = desc_sw128(sa), db = desc_sw128(sa + kTileBytes);
+                const uint32_t acc = tmem_base + buf * GN;
+                for (int kb = 0; kb < p.kb; ++kb, ++step) {
+                    const uint32_t st = step % kStages;
+                    if (!mbar_wait(b_full + 8 * st, (step / kStages) & 1, abort_flag)) {
+                        fail(2);
+                        ok = false;
+                        break;
+                    }
+                    fence_after();
+                    const uint32_t sa = s0 + st * kStageBytes;
+                    const uint64_t da = desc_sw128(sa), db = desc_sw128(sa + kTileBytes);
 #pragma unroll
-                for (int ks = 0; ks < kBK / kUK; ++ks)
-                    umma_bf16(tmem_base, da + 2 * ks, db + 2 * ks, kGemmIdesc,
-                              (kb | ks) != 0 ? 1u : 0u);
-                umma_commit(b_empty + 8 * st);
+                    for (int ks = 0; ks < kBK / kUK; ++ks)
+                        umma_bf16(acc, da + 2 * ks, db + 2 * ks, kGemmIdesc, (kb | ks) != 0 ? 1u : 0u);
+                    umma_commit(b_empty + 8 * st);
+                }
+                if (ok) umma_commit(b_tfull + 8 * buf);
             }
-            if (ok) umma_commit(b_tfull);
         }
     } else {
-        const int quarter = warp & 3;
-        if (mbar_wait(b_tfull, 0, abort_flag)) {
+        const int quarter = warp & 3, group = (warp - 2) >> 2;
+        uint32_t round = 0;
+        for (int64_t tile = first + group; tile < end; tile += kGroups, ++round) {
+            if (!mbar_wait(b_tfull + 8 * group, round & 1, abort_flag)) {
+                if (lane == 0) fail(3);
+                break;
+            }
             fence_after();
-            epilogue<EPI>(p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16),
-                          m0 + quarter * 32 + lane, n0, tile_n);
-        } else if (lane == 0) {
-            fail(3);
+            const int64_t tile_n = tile % p.n_tiles;
+            epilogue<EPI>(p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * GN,
+                          (tile / p.n_tiles) * GM + quarter * 32 + lane, tile_n * GN, tile_n,
+                          b_tempty + 8 * group);
         }
     }
 
@@ -260,20 +317,24 @@ __global__ void __launch_bounds__(192, 1)
     __syncthreads();
     if (warp == 1) {
         fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc(tmem_base, kGroups * GN);
     }
 }
 
-template <int EPI>
-void launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int64_t m_tiles,
-            cudaStream_t s) {
-    const size_t smem = static_cast<size_t>(kStages) * kStageBytes + 1024 + 128;
-    auto kern = gemm_kernel<EPI>;
+template <int EPI, int kGroups>
+void launch_groups(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t s) {
+    const size_t smem = static_cast<size_t>(kStages) * kStageBytes + 1024 + 256;
+    auto kern = gemm_kernel<EPI, kGroups>;
     UMAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     static_cast<int>(smem)));
-    const int64_t grid = m_tiles * p.n_tiles;
-    kern<<<static_cast<unsigned>(grid), 192, smem, s>>>(ma, mb, p);
+    kern<<<static_cast<unsigned>(ceil_div(p.tiles, p.per_cta)),
+           64 + 128 * kGroups, smem, s>>>(ma, mb, p);
     UMAPB_LAUNCH_CHECK();
+}
+
+template <int EPI>
+void launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t s) {
+    p.per_cta == 1 ? launch_groups<EPI, 1>(ma, mb, p, s) : launch_groups<EPI, 2>(ma, mb, p, s);
 }
 
 }  // namespace
@@ -295,15 +356,17 @@ void gemm_bf16_tn(const __nv_bfloat16* A, const __nv_bfloat16* B, int64_t M, int
     p.o = out;
     if (epilogue == kEpiRowMin && p.o.n_valid == 0) p.o.n_valid = N;
     const int64_t m_tiles = ceil_div(M, static_cast<int64_t>(GM));
-    if (m_tiles * p.n_tiles > 0x7FFFFFFFll) invalid("gemm_bf16_tn: too many tiles");
+    p.tiles = m_tiles * p.n_tiles;
+    p.per_cta = static_cast<int>(std::max<int64_t>(1, std::min(kMaxTilesPerCta, p.tiles / kTilesPerStep)));
+    if (p.tiles > 0x7FFFFFFFll) invalid("gemm_bf16_tn: too many tiles");
     const CUtensorMap ma = make_bf16_map(A, M, K, GM);
     const CUtensorMap mb = make_bf16_map(B, N, K, GN);
     switch (epilogue) {
-        case kEpiF32: launch<kEpiF32>(ma, mb, p, m_tiles, s); break;
-        case kEpiBiasGelu: launch<kEpiBiasGelu>(ma, mb, p, m_tiles, s); break;
-        case kEpiGeluBwd: launch<kEpiGeluBwd>(ma, mb, p, m_tiles, s); break;
-        case kEpiBiasGeluHead: launch<kEpiBiasGeluHead>(ma, mb, p, m_tiles, s); break;
-        case kEpiRowMin: launch<kEpiRowMin>(ma, mb, p, m_tiles, s); break;
+        case kEpiF32: launch<kEpiF32>(ma, mb, p, s); break;
+        case kEpiBiasGelu: launch<kEpiBiasGelu>(ma, mb, p, s); break;
+        case kEpiGeluBwd: launch<kEpiGeluBwd>(ma, mb, p, s); break;
+        case kEpiBiasGeluHead: launch<kEpiBiasGeluHead>(ma, mb, p, s); break;
+        case kEpiRowMin: launch<kEpiRowMin>(ma, mb, p, s); break;
         default: invalid("gemm_bf16_tn: unknown epilogue");
     }
 }
