@@ -895,18 +895,19 @@ void surrogate_transform_device(umapb_model* m, const float* Qd, int64_t nq, int
         flags = own.get();
     }
     const Surrogate& sg = *m->surrogate;
-    surrogate_gate_async(sg, Qd, nq, static_cast<int>(d), flags, s);
+    DevBuf<__nv_bfloat16> rows;  // freed on s after the network's stream has finished
+    surrogate_gate_async(sg, Qd, nq, static_cast<int>(d), flags, s, &rows);
     const int64_t nf = surrogate_count_flags(flags, nq, s);  // synchronises s
     if (n_fallback) *n_fallback = nf;
     if (!use_fallback || nf == 0) {
-        surrogate_forward_async(sg, Qd, nq, static_cast<int>(d), out, s);
+        surrogate_forward_async(sg, Qd, nq, static_cast<int>(d), out, s, &rows);
         surrogate_check(s);
         return;
     }
     SideWork net(m->side, 1);
     UMAPB_CUDA(cudaEventRecord(net.ready, s));
     UMAPB_CUDA(cudaStreamWaitEvent(net.s, net.ready, 0));
-    surrogate_forward_async(sg, Qd, nq, static_cast<int>(d), out, net.s);
+    surrogate_forward_async(sg, Qd, nq, static_cast<int>(d), out, net.s, &rows);
     UMAPB_CUDA(cudaEventRecord(net.done[0], net.s));
     surrogate_fallback(m, Qd, nq, d, out, flags, nf, -1, 0, net.done[0]);
     surrogate_check(net.s);

@@ -319,11 +319,13 @@ void surrogate_infer_async(const Surrogate& sg, const float* Q, int64_t nq, int 
                            uint8_t* flags, cudaStream_t s);
 // The gate alone (flags, no network outputs) and the network alone (outputs,
 // no gate), queued on `s` with no host wait; surrogate_check then waits for
-// `s` and reports a GEMM wait timeout.
+// `s` and reports a GEMM wait timeout.  The gate leaves the standardised rows
+// in `rows` where it takes them in one pass, and the network reads them there
+// instead of standardising once more; they must last until it is done.
 void surrogate_gate_async(const Surrogate& sg, const float* Q, int64_t nq, int d, uint8_t* flags,
-                          cudaStream_t s);
+                          cudaStream_t s, DevBuf<__nv_bfloat16>* rows = nullptr);
 void surrogate_forward_async(const Surrogate& sg, const float* Q, int64_t nq, int d, float* out,
-                             cudaStream_t s);
+                             cudaStream_t s, DevBuf<__nv_bfloat16>* rows = nullptr);
 void surrogate_check(cudaStream_t s);
 int64_t surrogate_count_flags(const uint8_t* flags, int64_t nq, cudaStream_t s);
 

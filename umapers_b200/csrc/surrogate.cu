@@ -150,6 +150,7 @@ __global__ void row_sq_bf16_kernel(const __nv_bfloat16* __restrict__ M, int64_t 
     const int lane = threadIdx.x & 31;
     if (r >= rows) return;
     float s = 0.0f;
+#pragma unroll 4
     for (int c = lane; c < cols; c += 32) {
         const float v = __bfloat162float(M[r * cols + c]);
         s = fmaf(v, v, s);
@@ -493,8 +494,12 @@ struct Pass {
     DevBuf<__nv_bfloat16> X, XT, A1, A1T, A2, dZ2, dZ2T, dZ1T;
     DevBuf<float> Z1, Z2, part, dY, y;
     void alloc(const Layout& L, int64_t n, bool train, cudaStream_t s) {
-        rows = n;
         X.alloc(n * L.dp, s);
+        alloc_network(L, n, train, s);
+    }
+    // all but the standardised rows
+    void alloc_network(const Layout& L, int64_t n, bool train, cudaStream_t s) {
+        rows = n;
         A1.alloc(n * L.H, s);
         part.alloc((L.H / 128) * n * L.dout, s);
         if (train) {
@@ -531,9 +536,9 @@ void standardize(const float* X, int d, const int32_t* ids, int64_t rows, const 
     UMAPB_LAUNCH_CHECK();
 }
 
-// Forward pass over P.rows rows already standardised into P.X; leaves the
-// head partial sums in P.part.  Training also keeps Z1, Z2, A1^T, A2.
-void forward(const Surrogate& sg, Pass& P, bool train, cudaStream_t s) {
+// Forward pass over the P.rows standardised rows X; leaves the head partial
+// sums in P.part.  Training also keeps Z1, Z2, A1^T, A2.
+void forward(const Surrogate& sg, Pass& P, const __nv_bfloat16* X, bool train, cudaStream_t s) {
     const Layout& L = sg.L;
     const float* w = sg.params.get();
     GemmOut o1;
@@ -544,7 +549,7 @@ void forward(const Surrogate& sg, Pass& P, bool train, cudaStream_t s) {
         o1.act_t = P.A1T.get();
         o1.ld_t = P.rows;
     }
-    gemm_bf16_tn(P.X.get(), sg.w1b.get(), P.rows, L.H, L.dp, kEpiBiasGelu, o1, s);
+    gemm_bf16_tn(X, sg.w1b.get(), P.rows, L.H, L.dp, kEpiBiasGelu, o1, s);
     GemmOut o2;
     o2.bias = w + L.b2;
     o2.head_w = w + L.w3;
@@ -671,11 +676,14 @@ void upload_vec(DevBuf<T>& dst, const std::vector<T>& v, cudaStream_t s) {
 // query rows Q[ids ? ids[r] : r].
 void infer_rows(const Surrogate& sg, const float* Q, const int32_t* ids, int64_t rows,
                 float* out, uint8_t* flags, int32_t* anchor_of, float* anchor_d2,
-                cudaStream_t s) {
+                cudaStream_t s, DevBuf<__nv_bfloat16>* kept = nullptr) {
     const Layout& L = sg.L;
     const int64_t chunk = std::min<int64_t>(rows, kInferChunk);
     Pass P;
-    P.alloc(L, chunk, false, s);
+    // the rows as an earlier call standardised them
+    const __nv_bfloat16* X = kept ? kept->get() : nullptr;
+    if (!X) P.X.alloc(chunk * L.dp, s);
+    if (out) P.alloc_network(L, chunk, false, s);
     // the gate runs only when its flags or nearest anchors are asked for
     const bool gate = sg.n_anchors > 0 && (flags || anchor_of || anchor_d2);
     const int a_tiles = gate ? static_cast<int>(ceil_div(sg.n_anchors, 128)) : 0;
@@ -689,16 +697,16 @@ void infer_rows(const Surrogate& sg, const float* Q, const int32_t* ids, int64_t
     for (int64_t r0 = 0; r0 < rows; r0 += chunk) {
         const int64_t n = std::min(chunk, rows - r0);
         P.rows = n;
-        if (ids)
+        if (!X && ids)
             standardize(Q, static_cast<int>(L.din), ids + r0, n, sg.mean.get(), sg.scale.get(),
                         static_cast<int>(L.dp), P.X.get(), nullptr, 0, s);
-        else
+        else if (!X)
             standardize(Q + r0 * L.din, static_cast<int>(L.din), nullptr, n, sg.mean.get(),
                         sg.scale.get(), static_cast<int>(L.dp), P.X.get(), nullptr, 0, s);
-        if (out) forward(sg, P, false, s);
+        const __nv_bfloat16* x = X ? X : P.X.get();
+        if (out) forward(sg, P, x, false, s);
         if (gate) {
-            row_sq_bf16_kernel<<<grid_for(n * 32), 256, 0, s>>>(P.X.get(), n,
-                                                                static_cast<int>(L.dp),
+            row_sq_bf16_kernel<<<grid_for(n * 32), 256, 0, s>>>(x, n, static_cast<int>(L.dp),
                                                                 row_sq.get());
             UMAPB_LAUNCH_CHECK();
             GemmOut og;
@@ -706,7 +714,7 @@ void infer_rows(const Surrogate& sg, const float* Q, const int32_t* ids, int64_t
             og.n_valid = sg.n_anchors;
             og.min_val = amin.get();
             og.min_idx = amin_idx.get();
-            gemm_bf16_tn(P.X.get(), sg.anchors.get(), n, sg.n_anchors, L.dp, kEpiRowMin, og, s);
+            gemm_bf16_tn(x, sg.anchors.get(), n, sg.n_anchors, L.dp, kEpiRowMin, og, s);
         }
         FinishArgs f{};
         f.head_part = P.part.get();
@@ -729,6 +737,7 @@ void infer_rows(const Surrogate& sg, const float* Q, const int32_t* ids, int64_t
         finish_kernel<<<grid_for(n), 256, 0, s>>>(f);
         UMAPB_LAUNCH_CHECK();
     }
+    if (kept && !X && rows <= kInferChunk) *kept = std::move(P.X);
 }
 
 double wall_now() {
@@ -863,7 +872,7 @@ SurrogatePtr surrogate_train(const float* X, int64_t n, int d, const float* emb,
             const int32_t* bid = perm.get() + st * B;
             standardize(X, d, bid, B, sg->mean.get(), sg->scale.get(), static_cast<int>(L.dp),
                         P.X.get(), P.XT.get(), B, s);
-            forward(*sg, P, true, s);
+            forward(*sg, P, P.X.get(), true, s);
             la.ids = bid;
             la.step = static_cast<uint64_t>(t);
             loss_kernel<<<grid_for(B), 256, 0, s>>>(la);
@@ -1021,17 +1030,17 @@ void surrogate_infer_async(const Surrogate& sg, const float* Q, int64_t nq, int 
 }
 
 void surrogate_gate_async(const Surrogate& sg, const float* Q, int64_t nq, int d, uint8_t* flags,
-                          cudaStream_t s) {
+                          cudaStream_t s, DevBuf<__nv_bfloat16>* rows) {
     if (d != sg.L.din) invalid("surrogate input width differs from the fitted rows");
     if (nq == 0) return;
-    infer_rows(sg, Q, nullptr, nq, nullptr, flags, nullptr, nullptr, s);
+    infer_rows(sg, Q, nullptr, nq, nullptr, flags, nullptr, nullptr, s, rows);
 }
 
 void surrogate_forward_async(const Surrogate& sg, const float* Q, int64_t nq, int d, float* out,
-                             cudaStream_t s) {
+                             cudaStream_t s, DevBuf<__nv_bfloat16>* rows) {
     if (d != sg.L.din) invalid("surrogate input width differs from the fitted rows");
     if (nq == 0) return;
-    infer_rows(sg, Q, nullptr, nq, out, nullptr, nullptr, nullptr, s);
+    infer_rows(sg, Q, nullptr, nq, out, nullptr, nullptr, nullptr, s, rows);
 }
 
 void surrogate_check(cudaStream_t s) { check_gemm(s); }
@@ -1109,7 +1118,7 @@ void mlp_grad(const umapb_mlp_batch& mb, float* grads, double* loss, float* y, c
     P.alloc(L, B, true, s);
     standardize(xd.get(), static_cast<int>(din), nullptr, B, sg.mean.get(), sg.scale.get(),
                 static_cast<int>(dp), P.X.get(), P.XT.get(), B, s);
-    forward(sg, P, true, s);
+    forward(sg, P, P.X.get(), true, s);
     LossArgs la{};
     la.head_part = P.part.get();
     la.n_tiles = static_cast<int>(H / 128);
