@@ -153,3 +153,39 @@ def test_orthonormalisation_at_its_chunk_edges(dim, m):
     # N(0, 1e-4) noise on every coordinate (6 sigma), FP32 products (6e-8)
     # over eigenvalue gaps of 4e-3 at a scale of 10
     assert np.abs(g - ref).max() < 6e-4 + 10 * 6e-8 / 4e-3 * 2
+
+
+# rows and features below, at and above the groups and tiles of the centroid sum
+@pytest.mark.parametrize("n_rows,d", [(5, 3), (15, 63), (16, 64), (17, 65), (100, 200)])
+def test_component_layout_follows_its_centroids(n_rows, d):
+    """Five rings of n_rows or n_rows + 1 rows.  A ring's own layout has mean
+    zero, so its mean is its place in the layout of the centroids: the second
+    and third eigenvectors of the normalised Laplacian of exp(-distance^2)."""
+    rng = np.random.default_rng(n_rows)
+    h, t, x = [], [], []
+    base = 0
+    size = [n_rows + c % 2 for c in range(5)]
+    centre = rng.standard_normal((5, d))
+    centre *= 0.9 / np.linalg.norm(centre, axis=1, keepdims=True)
+    for c, m in enumerate(size):
+        i = np.arange(m)
+        h += [base + i, base + (i + 1) % m]
+        t += [base + (i + 1) % m, base + i]
+        x.append((rng.standard_normal((m, d)) * 0.3 + centre[c]).astype(np.float32))
+        base += m
+    h, t = np.concatenate(h), np.concatenate(t)
+    order = np.lexsort((t, h))
+    g, used = gu.spectral_init(np.concatenate(x), h[order].astype(np.int32),
+                               t[order].astype(np.int32), np.ones(h.size, np.float32), 2, 42)
+    assert used
+    mid = np.array([p.mean(0) for p in np.split(g.astype(np.float64), np.cumsum(size)[:-1])])
+    cent = np.array([p.astype(np.float64).mean(0) for p in x])
+    aff = np.exp(-((cent[:, None] - cent[None]) ** 2).sum(-1))
+    deg = aff.sum(1)
+    val, vec = np.linalg.eigh(np.eye(5) - aff / np.sqrt(deg[:, None] * deg[None]))
+    assert np.diff(val)[:3].min() > 1e-3
+    ref = vec[:, 1:3] * (10.0 / np.abs(vec[:, 1:3]).max())
+    ref *= np.sign((ref * mid).sum(0))
+    # N(0, 1e-4) noise on the places and on the rows (6 sigma each), FP32
+    # coordinates near 10 and their mean (6e-8 each)
+    assert np.abs(mid - ref).max() < 1.2e-3 + 4 * 10 * 6e-8
