@@ -9,8 +9,9 @@
 // index, cut to max_candidates by a random partial Fisher-Yates shuffle, all
 // evaluated, best k kept by (distance, index).  Iterations read the previous
 // lists and write new ones (as the reference's collect-then-replace does) and
-// stop when no row changed.  One warp owns one row; candidates live in shared
-// memory and are ordered with warp bitonic sorts.  Distances use the
+// stop when no row changed.  One warp owns one row; candidates live in its
+// registers for k <= 31, else in shared memory, and are ordered with warp
+// bitonic sorts.  Distances use the
 // reference's summation order (euclidean = sqrt of the squared distance,
 // lib.rs:3167).  Random streams are counter-based per (row, iteration).
 //

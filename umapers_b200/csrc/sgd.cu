@@ -15,9 +15,10 @@
 // deterministic layout of sgd_small.cu instead.
 //
 // transform_layout: init_graph_transform (lib.rs:4793-4836) followed by
-// optimize_layout_transform (lib.rs:5444-5544).  Queries never interact, so
-// one thread runs one query's whole schedule sequentially, as the reference's
-// per-query closure does.
+// optimize_layout_transform (lib.rs:5444-5544).  Queries never interact, so a
+// query's whole schedule runs sequentially, as in the reference's per-query
+// closure: on one thread, or for few queries on 4 to 16 lanes of which one
+// updates and the others fetch ahead.
 #include <cub/cub.cuh>
 
 #include <cfloat>
