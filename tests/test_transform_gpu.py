@@ -69,3 +69,25 @@ def test_transform_does_not_depend_on_the_lanes_per_query(k, rate):
     for n in (1, 31, 700, 4096, 4097, 8193):
         whole = np.tile(q[:n], (16385 // n + 1, 1))
         assert np.array_equal(m.transform(q[:n]), m.transform(whole)[:n])
+
+
+@pytest.mark.parametrize("n", [1, 4097, 8193, 16385])
+def test_transform_device_writes_to_any_float_address(n):
+    # 16, 8 and 4 lanes a query and one thread a query: the same positions in
+    # an array that starts one float off a vector boundary, nothing around it
+    import torch
+
+    from umapers_b200 import _lib
+
+    fit, q = workloads.transform_mixture(n_fit=1000, n_query=n, d=16, n_comp=4)
+    m = Umap(n_neighbors=10, n_epochs=10, random_seed=5)
+    m.fit(fit)
+    qd = torch.from_numpy(q).cuda()
+    flat = torch.full((2 * n + 3,), -7.0, device="cuda")
+    assert flat.data_ptr() % 8 == 0
+    want = torch.empty((n, 2), device="cuda")
+    torch.cuda.synchronize()
+    for out in (want.data_ptr(), flat.data_ptr() + 4):
+        _lib.check(_lib.load().umapb_transform_device(m._core._handle, qd.data_ptr(), n, 16, out))
+    assert torch.equal(flat[1:-2].reshape(n, 2), want)
+    assert flat[0] == -7.0 and (flat[-2:] == -7.0).all()

@@ -996,7 +996,9 @@ __global__ void __launch_bounds__(kTransformThreads) transform_group_kernel(Tran
             init_query(p, st, en, c2);
             transform_schedule_2d(p, q, st, en, qseed, c2);
         }
-        reinterpret_cast<float2*>(p.out)[q] = make_float2(c2[0], c2[1]);
+        // a caller's device array: any float address
+        p.out[q * 2] = c2[0];
+        p.out[q * 2 + 1] = c2[1];
     }
 }
 
