@@ -127,3 +127,15 @@ def test_large_csr_faults_are_named_in_row_order(faults, message):
     core = UmapCore(n_neighbors=5, n_components=2)
     with pytest.raises(Exception, match=message):
         core.transform_sparse_csr(ip, ix, dv, n_cols)
+
+
+# below and at the bound: an error of the call, after which the next one works
+@pytest.mark.parametrize("n", [1000, STAGED // 64 - 1, STAGED // 64, STAGED // 32])
+def test_a_null_array_is_an_error(n):
+    lib, k = _lib.load(), 3
+    r = np.random.default_rng(0).standard_normal((50, 16), np.float32)
+    idx, dist = np.empty((n, k), np.int64), np.empty((n, k), np.float32)
+    assert lib.umapb_knn_exact(None, n, 16, k, 0, 0, gu._p(idx), gu._p(dist), None) != 0
+    assert lib.umapb_knn_query(None, n, gu._p(r), 50, 16, k, 0, 0, gu._p(idx), gu._p(dist)) != 0
+    assert lib.umapb_knn_query(gu._p(r), 50, None, n, 16, k, 0, 0, gu._p(idx), gu._p(dist)) != 0
+    _self_neighbours(r, np.arange(50))

@@ -168,6 +168,8 @@ int host_threads() {
 
 void upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s) {
     if (bytes == 0) return;
+    // an error of the call, as cudaMemcpyAsync makes it: staging would read it
+    if (!src) throw_cuda(cudaErrorInvalidValue, "upload of a null host array", __FILE__, __LINE__);
     const int threads = host_threads();
     if (bytes >= kStagedBytes && threads > 1 && pageable(src)) {
         StageLease lease;
