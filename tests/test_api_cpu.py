@@ -3,6 +3,9 @@ normalisation and the reference's validation errors, which all fire before
 any device work.  Mirrors umap_rs/tests/test_binding.py and the error
 contracts of rust_umap/src/lib.rs tests."""
 import inspect
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -246,3 +249,54 @@ def test_umapcore_is_importable_from_the_drop_in_path():
     assert core.n_neighbors == 12 and core.n_components == 3 and core.n_features is None
     assert core.embedding is None
     assert umapers.__version__.startswith("1.")
+
+
+@pytest.mark.parametrize("indptr,indices,message", [
+    ([0, 10 ** 6, 5], [0, 1, 2, 3, 4], "csr indptr must be non-decreasing, got "
+                                       "indptr[1]=1000000 > indptr[2]=5"),
+    ([0, 3, 6, 5], [0, 1, 2, 0, 1], "csr indptr must be non-decreasing, got "
+                                    "indptr[2]=6 > indptr[3]=5"),
+    ([0, 2, 7, 9, 9, 4, 5], [0, 1, 2, 3, 4], "csr indptr must be non-decreasing, got "
+                                             "indptr[4]=9 > indptr[5]=4"),
+    ([0, 2, -1], [], "csr indptr must be non-decreasing, got indptr[1]=2 > indptr[2]=-1"),
+    # rows ahead of the bad offset keep their faults
+    ([0, 2, 10 ** 6, 5], [3, 3, 0, 1, 2], "csr row 0 indices must be strictly increasing"),
+    ([0, 2, 10 ** 6, 5], [3, 9, 0, 1, 2], "csr row 0 has column index 9 out of bounds"),
+    ([0, 2, 1, 5], [0, 1, 0, 1, 2], "csr indptr must be non-decreasing, got "
+                                    "indptr[1]=2 > indptr[2]=1"),
+])
+def test_csr_offsets_past_the_stored_entries_are_named_without_reading_there(indptr, indices,
+                                                                             message):
+    # the arrays end where memory that cannot be read begins
+    code = f"""
+import ctypes, mmap
+import numpy as np
+from umapers_b200 import _lib
+
+def ending_at_a_guard(a):
+    size = mmap.mmap(-1, 2 * mmap.PAGESIZE)
+    base = np.frombuffer(size, np.uint8).ctypes.data
+    libc = ctypes.CDLL(None)
+    assert libc.mprotect(ctypes.c_void_p(base + mmap.PAGESIZE), mmap.PAGESIZE, 0) == 0
+    at = base + mmap.PAGESIZE - a.nbytes
+    ctypes.memmove(at, a.ctypes.data, a.nbytes)
+    keep.append(size)
+    return at
+
+keep = []
+ip = np.array({indptr}, np.int64)
+ix, dv = np.array({indices}, np.int64), np.ones({len(indices)}, np.float32)
+lib, p, h = _lib.load(), _lib.Params(), ctypes.c_void_p()
+lib.umapb_params_default(ctypes.byref(p))
+assert lib.umapb_create(ctypes.byref(p), ctypes.byref(h)) == 0
+try:
+    _lib.check(lib.umapb_fit_csr(h, ip.ctypes.data, ending_at_a_guard(ix), ending_at_a_guard(dv),
+                                 len(ip) - 1, 8))
+except ValueError as e:
+    print(e, flush=True)
+import os
+os._exit(0)
+"""
+    got = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                         cwd=Path(__file__).resolve().parents[1])
+    assert got.returncode == 0 and message in got.stdout, (got.returncode, got.stdout, got.stderr)

@@ -179,8 +179,8 @@ void validate_csr_host(const int64_t* indptr, const int64_t* indices, const floa
     if (!indptr || (indptr[n_rows] > 0 && (!indices || !data))) invalid("null csr array");
     if (indptr[0] != 0) invalid("csr indptr must start from 0");
     // Entries [0, nnz) in ranges over threads, of whole rows; where one finds a
-    // fault, the rows are walked in order for the first of them.  The offsets
-    // come before anything that they index.
+    // fault, the rows are walked in order for the first of them.  No entry at or
+    // past nnz is read: an offset above nnz means that a later one decreases.
     const int64_t nnz = indptr[n_rows];
     bool ordered = true;
     for (int64_t row = 0; row < n_rows; ++row) ordered &= indptr[row] <= indptr[row + 1];
@@ -210,10 +210,12 @@ void validate_csr_host(const int64_t* indptr, const int64_t* indices, const floa
         });
     if (!good) {
         for (int64_t row = 0; row < n_rows; ++row) {
-            if (indptr[row] > indptr[row + 1])
+            if (indptr[row] > indptr[row + 1] || indptr[row + 1] > nnz) {
+                while (indptr[row] <= indptr[row + 1]) ++row;
                 invalid("csr indptr must be non-decreasing, got indptr[" + std::to_string(row) +
                         "]=" + std::to_string(indptr[row]) + " > indptr[" + std::to_string(row + 1) +
                         "]=" + std::to_string(indptr[row + 1]));
+            }
             for (int64_t e = indptr[row] + 1; e < indptr[row + 1]; ++e)
                 if (indices[e - 1] >= indices[e])
                     invalid("csr row " + std::to_string(row) + " indices must be strictly increasing");
