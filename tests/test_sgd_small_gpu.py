@@ -108,3 +108,15 @@ def test_small_layout_matches_sequential_replay(n, dim, deg, n_epochs, rate):
     k = (np.bincount(h, minlength=n) * (1 + rate) + np.bincount(t, minlength=n)) * (n_epochs - 1)
     bound = 2 * k * 4 * lr * 5e-5 + 1e-6 * np.abs(emb).max()
     assert (np.abs(got - ref).max(1) <= bound).all()
+
+
+def test_an_event_may_wait_longer_than_the_limit_on_idle_polls():
+    # Two edges with one head: the second waits for the first one's 8,000,000
+    # negatives, 1.5 s, longer than the limit on polls without any update.
+    # Vertex 3 has no edge, and every point must stay finite and have moved.
+    h, t = np.array([0, 0], np.int32), np.array([1, 2], np.int32)
+    emb = np.random.default_rng(0).normal(0, 3, (4, 2)).astype(np.float32)
+    got = optimize_layout(emb, h, t, np.ones(2, np.float32), 2, 1.577, 0.895, neg_rate=8_000_000,
+                          seed=3)
+    assert np.isfinite(got).all() and np.array_equal(got[3], emb[3])
+    assert (got[:3] != emb[:3]).any(1).all()

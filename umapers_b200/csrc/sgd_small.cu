@@ -44,7 +44,11 @@
 //
 // A wait always ends: batches are in an order that respects the dependencies
 // and a warp takes its own in that order, so the first batch that is not done
-// waits only for batches that are.  It is bounded all the same (kSpinLimit).
+// waits only for batches that are.  It is bounded all the same: a warp stops
+// the layout after kSpinLimit polls during which no warp of the CTA has got any
+// further (the vertices' counts, and `beat` within a long run of negatives).
+// How long a batch may wait has no bound of its own: at a negative rate of
+// 8,000,000 one event takes 1.5 s.
 #include <algorithm>
 #include <vector>
 
@@ -62,7 +66,7 @@ constexpr uint32_t kNotDue = 0xffffffffu;
 constexpr int kInlineNeg = 14;      // negatives stored in the event (rate 5 draws 3 to 9)
 constexpr int kStartBuckets = 4096;  // distinct start times an epoch is sorted by
 constexpr uint32_t kByColor = 0x80000000u;  // flag on n_batches: the events are in colour order
-constexpr uint32_t kSpinLimit = 1u << 23;  // fruitless polls (about 0.5 s)
+constexpr uint32_t kSpinLimit = 1u << 23;  // polls while no warp updates anything (about 1 s)
 constexpr size_t kBlockBytes = static_cast<size_t>(256) << 20;  // work space of one block of epochs
 constexpr size_t kBlockStep = static_cast<size_t>(32) << 20;
 constexpr int64_t kBlockEpochs = 148;  // one order_kernel CTA per SM
@@ -355,6 +359,12 @@ struct Vertices {
                                  : "memory");
         }
     }
+    __device__ __forceinline__ uint32_t count(uint32_t v) const {
+        const uint32_t word = D == 1 ? v * 2 + 1 : kPacked ? v * 4 + 3 : n * dim + v;
+        uint32_t c;
+        asm volatile("ld.relaxed.cta.shared::cta.u32 %0, [%1];" : "=r"(c) : "r"(at + word * 4) : "memory");
+        return c;
+    }
     __device__ __forceinline__ void store(uint32_t v, const float* pos, uint32_t count) const {
         if constexpr (D == 1) {
             const uint64_t w = static_cast<uint64_t>(count) << 32 | __float_as_uint(pos[0]);
@@ -393,6 +403,7 @@ template <int D>
 __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
     extern __shared__ __align__(16) float lsm[];
     __shared__ int stop;
+    __shared__ uint32_t beat;  // moves on with every 1,024 negatives of an event
     __shared__ uint32_t counts[kBlockEpochs];
     constexpr int kD = Vertices<D>::kD;
     const int dim = D > 0 ? D : p.dim;
@@ -411,8 +422,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
     for (uint32_t v = tid; v < nv; v += kSmallThreads) verts.store(v, snap + v * dim, 0);
     for (int b = tid; b < p.n_block; b += kSmallThreads) counts[b] = p.n_batches[b];
     if (tid == 0) stop = 0;
+    if (tid == 0) beat = 0;
     __syncthreads();
     const float nef = static_cast<float>(p.n_epochs);
+    auto reached = [&] {  // moves on whenever a warp gets further within an epoch
+        uint32_t sum = lane == 0 ? *static_cast<volatile uint32_t*>(&beat) : 0u;
+        for (uint32_t v = lane; v < nv; v += 32) sum += verts.count(v);
+        return __reduce_add_sync(0xffffffffu, sum);
+    };
 
     for (int b = 0; b < p.n_block; ++b) {
         const int n_batches = static_cast<int>(counts[b] & ~kByColor);
@@ -464,7 +481,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                 const uint32_t w[7] = {e1.y, e1.z, e1.w, e2.x, e2.y, e2.z, e2.w};
                 return (s & 1) ? w[s >> 1] >> 16 : w[s >> 1] & 0xffffu;
             };
-            uint32_t idle = 0;
+            uint32_t idle = 0, seen = ~0u;
             while (todo) {
                 bool ready = false;
                 float h[kD], t[kD];
@@ -481,13 +498,19 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                 }
                 todo &= ~now;
                 if (now == 0) {
-                    if ((++idle & 1023u) == 0 &&
-                        __any_sync(0xffffffffu,
-                                   idle > kSpinLimit || *static_cast<volatile int*>(&stop))) {
-                        *static_cast<volatile int*>(&stop) = 1;
-                        *p.err = 1;
-                        j = n_batches;
-                        break;
+                    if ((++idle & 1023u) == 0) {
+                        if (idle > kSpinLimit) {
+                            const uint32_t at = reached();
+                            if (at != seen) idle = 0;
+                            seen = at;
+                        }
+                        if (__any_sync(0xffffffffu,
+                                       idle > kSpinLimit || *static_cast<volatile int*>(&stop))) {
+                            *static_cast<volatile int*>(&stop) = 1;
+                            *p.err = 1;
+                            j = n_batches;
+                            break;
+                        }
                     }
                     continue;
                 }
@@ -544,6 +567,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                         if (s + 1 == n_neg) verts.store(head, h, rank_h + 1);
                     }
                     for (uint32_t s = kInlineNeg; s < n_neg; ++s) {
+                        if ((s & 1023u) == 0) {
+                            volatile uint32_t* const at = &beat;
+                            *at = *at + 1;
+                        }
                         const uint64_t word =
                             rng_word(p.seed, e1.x, (static_cast<uint64_t>(epoch) << 32) | s);
                         const uint32_t v = rng_below(word, nv);
