@@ -120,3 +120,10 @@ def test_an_event_may_wait_longer_than_the_limit_on_idle_polls():
                           seed=3)
     assert np.isfinite(got).all() and np.array_equal(got[3], emb[3])
     assert (got[:3] != emb[:3]).any(1).all()
+
+
+# positions wider than a word, polled by their counter alone: the first and the
+# last such width, and the most vertices of the last
+@pytest.mark.parametrize("n,dim,deg", [(200, 5, 3), (200, 9, 3), (200, 16, 3), (1024, 16, 1)])
+def test_wide_positions_match_sequential_replay(n, dim, deg):
+    test_small_layout_matches_sequential_replay(n, dim, deg, 3, 5)

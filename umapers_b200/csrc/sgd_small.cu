@@ -346,18 +346,31 @@ struct Vertices {
             if constexpr (D == 3) pos[2] = __uint_as_float(static_cast<uint32_t>(hi));
             count = static_cast<uint32_t>(hi >> 32);
         } else {
+            poll(v, pos, count);
+            fetch(v, pos);
+        }
+    }
+    // What a waiting warp reads again and again: the counter, with the position
+    // where both are one word.  Wider positions are fetched once the counter is
+    // right: with every poll they filled the shared-memory pipe that the
+    // working warps need.
+    __device__ __forceinline__ void poll(uint32_t v, float* pos, uint32_t& count) const {
+        if constexpr (kPacked)
+            load(v, pos, count);
+        else
             asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];"
                          : "=r"(count)
                          : "r"(at + (n * dim + v) * 4)
                          : "memory");
+    }
+    __device__ __forceinline__ void fetch(uint32_t v, float* pos) const {
 #pragma unroll
-            for (int d = 0; d < kD; ++d)
-                if (D > 0 || d < static_cast<int>(dim))
-                    asm volatile("ld.relaxed.cta.shared::cta.f32 %0, [%1];"
-                                 : "=f"(pos[d])
-                                 : "r"(at + (v * dim + d) * 4)
-                                 : "memory");
-        }
+        for (int d = 0; d < kD; ++d)
+            if (D > 0 || d < static_cast<int>(dim))
+                asm volatile("ld.relaxed.cta.shared::cta.f32 %0, [%1];"
+                             : "=f"(pos[d])
+                             : "r"(at + (v * dim + d) * 4)
+                             : "memory");
     }
     __device__ __forceinline__ uint32_t count(uint32_t v) const {
         const uint32_t word = D == 1 ? v * 2 + 1 : kPacked ? v * 4 + 3 : n * dim + v;
@@ -487,8 +500,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                 float h[kD], t[kD];
                 if ((todo >> lane) & 1u) {
                     uint32_t ch, ct;
-                    verts.load(head, h, ch);
-                    verts.load(tail, t, ct);
+                    verts.poll(head, h, ch);
+                    verts.poll(tail, t, ct);
                     ready = ch == rank_h && (ct == rank_t || head == tail);
                 }
                 unsigned now = __ballot_sync(0xffffffffu, ready);
@@ -515,6 +528,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                     continue;
                 }
                 if (ready) {
+                    if constexpr (!Vertices<D>::kPacked) {
+                        verts.fetch(head, h);
+                        verts.fetch(tail, t);
+                    }
                     {
                         float d2 = 0.0f;
                         each([&](int d) {
