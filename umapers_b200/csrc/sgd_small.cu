@@ -67,6 +67,7 @@ constexpr int kInlineNeg = 14;      // negatives stored in the event (rate 5 dra
 constexpr int kStartBuckets = 4096;  // distinct start times an epoch is sorted by
 constexpr uint32_t kByColor = 0x80000000u;  // flag on n_batches: the events are in colour order
 constexpr uint32_t kSpinLimit = 1u << 23;  // polls while no warp updates anything (about 1 s)
+constexpr uint32_t kBeatEvery = 4096;      // negatives
 constexpr size_t kBlockBytes = static_cast<size_t>(256) << 20;  // work space of one block of epochs
 constexpr size_t kBlockStep = static_cast<size_t>(32) << 20;
 constexpr int64_t kBlockEpochs = 148;  // one order_kernel CTA per SM
@@ -416,7 +417,7 @@ template <int D>
 __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
     extern __shared__ __align__(16) float lsm[];
     __shared__ int stop;
-    __shared__ uint32_t beat;  // moves on with every 1,024 negatives of an event
+    __shared__ uint32_t beat;  // moves on with every kBeatEvery negatives of an event
     __shared__ uint32_t counts[kBlockEpochs];
     constexpr int kD = Vertices<D>::kD;
     const int dim = D > 0 ? D : p.dim;
@@ -583,17 +584,18 @@ __global__ void __launch_bounds__(kSmallThreads, 1) layout_kernel(SmallArgs p) {
                         // a lane frees its head as soon as its own negatives are done
                         if (s + 1 == n_neg) verts.store(head, h, rank_h + 1);
                     }
-                    for (uint32_t s = kInlineNeg; s < n_neg; ++s) {
-                        if ((s & 1023u) == 0) {
-                            volatile uint32_t* const at = &beat;
-                            *at = *at + 1;
+                    for (uint32_t s = kInlineNeg; s < n_neg;) {
+                        const uint32_t end = min(n_neg, s + kBeatEvery);
+                        for (; s < end; ++s) {
+                            const uint64_t word =
+                                rng_word(p.seed, e1.x, (static_cast<uint64_t>(epoch) << 32) | s);
+                            const uint32_t v = rng_below(word, nv);
+                            each([&](int d) { o[d] = snap[v * dim + d]; });
+                            repel(o, v != head);
+                            if (s + 1 == n_neg) verts.store(head, h, rank_h + 1);
                         }
-                        const uint64_t word =
-                            rng_word(p.seed, e1.x, (static_cast<uint64_t>(epoch) << 32) | s);
-                        const uint32_t v = rng_below(word, nv);
-                        each([&](int d) { o[d] = snap[v * dim + d]; });
-                        repel(o, v != head);
-                        if (s + 1 == n_neg) verts.store(head, h, rank_h + 1);
+                        volatile uint32_t* const at = &beat;
+                        *at = *at + 1;
                     }
                 }
                 __syncwarp();  // the next polls see these updates
