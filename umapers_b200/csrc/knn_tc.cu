@@ -1187,8 +1187,7 @@ template <int MT, int BN, bool SA>
 void launch_tc_t(const SideMaps& ma, const SideMaps& mb, const TcArgs& a, size_t smem,
                  cudaStream_t s) {
     auto kern = tc_knn_kernel<MT, BN, SA>;
-    UMAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
+    allow_shared(kern);
     int dev = 0, sms = 0;
     UMAPB_CUDA(cudaGetDevice(&dev));
     UMAPB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1366,8 +1365,7 @@ void launch_assign(const float* X, int64_t n, int d, uint8_t* cell, int32_t* iot
     constexpr int C = 32 * PPL;
     const size_t smem = (static_cast<size_t>(C) * d + C) * sizeof(float);
     auto kern = cell_assign_kernel<PPL>;
-    UMAPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
+    allow_shared(kern);
     int dev = 0, sms = 0;
     UMAPB_CUDA(cudaGetDevice(&dev));
     UMAPB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -701,9 +701,7 @@ int64_t nndescent_run(NdArgs p, int64_t n, int k, int64_t n_iters, size_t smem, 
     UMAPB_CUDA(cudaMemsetAsync(evaluated.get(), 0, kEvalSlots * 8, s));
     p.evaluated = evaluated.get();
     p.changed = changed.get();
-    UMAPB_CUDA(cudaFuncSetAttribute(nd_init_kernel<SP>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(smem)));
+    allow_shared(nd_init_kernel<SP>);
     const unsigned grid = static_cast<unsigned>(ceil_div(n, kWarps));
     // k <= 31 keeps the candidates in registers (row indices below 2^31, k
     // best within one warp's list); longer lists take the shared-memory form
@@ -722,8 +720,7 @@ int64_t nndescent_run(NdArgs p, int64_t n, int k, int64_t n_iters, size_t smem, 
         if (iterate != nd_iter_kernel<SP>)
             iter_smem = kWarps * nd_reg_smem<SP>(p.cap, SP ? p.csr.max_nnz : p.d);
     }
-    UMAPB_CUDA(cudaFuncSetAttribute(iterate, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(iter_smem)));
+    allow_shared(iterate);
     int32_t* cur_i = out_idx;
     float* cur_d = out_dist;
     int32_t* nxt_i = idx_b.get();
