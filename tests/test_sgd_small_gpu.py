@@ -2,9 +2,15 @@
 edges coloured greedily in graph order, each epoch's due edges one after
 another by (colour, graph order), negatives from the epoch's starting
 positions (rust_umap/src/lib.rs:5172-5318 per edge)."""
+import ctypes
+import gc
+import threading
+
 import numpy as np
 import pytest
 
+from umapers import Umap
+from umapers_b200 import _lib
 from tests.gpu_util import optimize_layout
 
 pytestmark = pytest.mark.gpu
@@ -127,3 +133,48 @@ def test_an_event_may_wait_longer_than_the_limit_on_idle_polls():
 @pytest.mark.parametrize("n,dim,deg", [(200, 5, 3), (200, 9, 3), (200, 16, 3), (1024, 16, 1)])
 def test_wide_positions_match_sequential_replay(n, dim, deg):
     test_small_layout_matches_sequential_replay(n, dim, deg, 3, 5)
+
+
+def _fit(x, seed):
+    m = Umap(n_neighbors=15, n_epochs=200, random_seed=seed)
+    return m, m.fit_transform(x)
+
+
+def test_models_alive_share_the_work_space():
+    # 1,000 rows of 32 columns ask for 224 MB of it, and for about 1 MB else
+    lib = _lib.load()
+    reserved, used = ctypes.c_int64(0), ctypes.c_int64(0)
+
+    def pool():
+        _lib.check(lib.umapb_pool_bytes(ctypes.byref(reserved), ctypes.byref(used)))
+        return used.value
+
+    x = np.random.default_rng(0).normal(size=(1000, 32)).astype(np.float32)
+    before = pool()
+    models = [_fit(x, 1)]
+    one = pool()
+    models += [_fit(x, 1) for _ in range(4)]
+    assert one - before <= 272 << 20 and pool() - one <= 4 * (16 << 20)
+    assert all(np.array_equal(e, models[0][1]) for _, e in models)
+    models.clear()
+    gc.collect()
+    assert pool() <= before + (256 << 20)  # models of other tests may be alive
+
+
+def test_fits_of_several_threads_keep_their_work_spaces_apart():
+    rng = np.random.default_rng(1)
+    data = [rng.normal(size=(n, 16)).astype(np.float32) for n in (300, 900, 1500, 2400)]
+    want = [_fit(x, 7)[1] for x in data]
+    got = [[] for _ in data]
+
+    def work(i):
+        for _ in range(3):
+            got[i].append(_fit(data[i], 7)[1])
+
+    team = [threading.Thread(target=work, args=(i,)) for i in range(len(data))]
+    for t in team:
+        t.start()
+    for t in team:
+        t.join()
+    for g, w in zip(got, want):
+        assert len(g) == 3 and all(np.array_equal(e, w) for e in g)

@@ -19,6 +19,7 @@
 namespace umapb {
 
 extern std::atomic<unsigned long long> g_kernel_launches;
+extern std::atomic<int64_t> g_models;  // alive
 
 // A failed call carries a umapb_status and the user-facing message.
 struct Error : public std::runtime_error {
@@ -80,12 +81,19 @@ void allow_shared(Kernel* kernel) {
 // stream).  Blocks of a stream that is gone stay until the process ends,
 // within the same limit.  An allocation the pool cannot serve returns every
 // block kept for the device and is tried once more.
+//
+// `spare` is one more block, for work space that is large beside a small
+// model's data and needed only during a call: whichever call is next takes it,
+// on any stream, so many models alive hold it once and not once each.
 constexpr size_t kBlockCacheBytes = static_cast<size_t>(32) << 30;
 
 struct BlockCache {
     std::mutex mu;
     std::map<std::tuple<int, cudaStream_t, size_t>, std::vector<void*>> free_blocks;
     size_t held = 0;
+    void* spare = nullptr;  // no work of any stream uses it
+    size_t spare_bytes = 0;
+    int spare_dev = 0;
     static BlockCache& get() {
         static BlockCache c;
         return c;
@@ -122,6 +130,10 @@ inline void* dev_alloc(size_t bytes, cudaStream_t s, int* dev_out) {
                 } else {
                     ++it;
                 }
+            }
+            if (c.spare && c.spare_dev == dev) {
+                blocks.push_back(c.spare);
+                c.spare = nullptr;
             }
         }
         if (!blocks.empty()) {
@@ -166,6 +178,55 @@ inline void dev_release_stream(cudaStream_t s) {
         }
     }
     for (void* p : blocks) cudaFreeAsync(p, s);
+}
+
+// Work space of one call on stream `s`: the spare block where it is large
+// enough, else a new one.  keep(), once the stream has been waited for, makes it
+// the spare block while a model is alive; otherwise it goes back to the pool.
+struct WorkBlock {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    cudaStream_t stream = nullptr;
+    int device = 0;
+
+    WorkBlock(size_t want, cudaStream_t s) : bytes(want), stream(s) {
+        cudaGetDevice(&device);
+        BlockCache& c = BlockCache::get();
+        {
+            std::lock_guard<std::mutex> lk(c.mu);
+            if (c.spare && c.spare_dev == device && c.spare_bytes >= want) {
+                ptr = c.spare;
+                bytes = c.spare_bytes;
+                c.spare = nullptr;
+            }
+        }
+        if (!ptr) ptr = dev_alloc(want, s, &device);
+    }
+    ~WorkBlock() {
+        if (ptr) cudaFreeAsync(ptr, stream);
+    }
+    void keep(size_t most) {
+        BlockCache& c = BlockCache::get();
+        std::lock_guard<std::mutex> lk(c.mu);
+        if (g_models.load() == 0 || bytes > most) return;
+        if (c.spare && (c.spare_dev != device || c.spare_bytes >= bytes)) return;
+        std::swap(ptr, c.spare);  // a smaller one goes back to the pool
+        c.spare_bytes = bytes;
+        c.spare_dev = device;
+    }
+    WorkBlock(const WorkBlock&) = delete;
+    WorkBlock& operator=(const WorkBlock&) = delete;
+};
+
+// Returns the spare block; called when no model is left.
+inline void dev_release_spare() {
+    BlockCache& c = BlockCache::get();
+    void* p = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(c.mu);
+        std::swap(p, c.spare);
+    }
+    if (p) cudaFree(p);
 }
 
 // Stream-ordered device buffer on the block cache above (backed by the

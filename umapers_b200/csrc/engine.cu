@@ -22,6 +22,7 @@
 
 namespace umapb {
 std::atomic<unsigned long long> g_kernel_launches{0};
+std::atomic<int64_t> g_models{0};
 }  // namespace umapb
 
 using namespace umapb;
@@ -29,7 +30,6 @@ using namespace umapb;
 namespace {
 
 thread_local std::string g_last_error;
-std::atomic<int64_t> g_models{0};  // alive
 
 constexpr const char* kVersion = "1.1.4+b200.1";
 constexpr float kSmoothKTolerance = 1e-5f;  // lib.rs:19
@@ -1054,7 +1054,7 @@ void destroy_model(umapb_model* m) {
         }
     }
     delete m;
-    g_models.fetch_sub(1);
+    if (g_models.fetch_sub(1) == 1) dev_release_spare();
 }
 }  // namespace
 

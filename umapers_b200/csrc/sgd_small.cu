@@ -671,9 +671,12 @@ double optimize_layout_small(float* emb, int64_t n_vertices, int dim, const Grap
                               (batch_cap + 1) * static_cast<int64_t>(sizeof(uint32_t));
     const int64_t block = std::max<int64_t>(
         1, std::min({n_epochs, kBlockEpochs, static_cast<int64_t>(kBlockBytes) / per_epoch}));
-    // the work space in whole steps of kBlockStep, so that graphs of like size
-    // ask for the same block
-    DevBuf<uint8_t> work(ceil_div(block * per_epoch, static_cast<int64_t>(kBlockStep)) * kBlockStep, s);
+    // The work space in whole steps of kBlockStep, so that graphs of like size
+    // ask for the same block.  It is not the model's: 1,000 rows take 224 MB of
+    // it for 148 epochs, and a new block of that size costs 3 ms.  Fewer epochs at
+    // a time would need less, but every block's order_kernel (0.2 to 0.5 ms)
+    // comes before its layout.
+    WorkBlock work(ceil_div(block * per_epoch, static_cast<int64_t>(kBlockStep)) * kBlockStep, s);
     DevBuf<int32_t> dorder(m, s), dh(m, s), dt(m, s), dptr(n_colors + 1, s);
     DevBuf<float> deps(m, s), dnext(m, s), dneg(m, s);
     DevBuf<unsigned long long> samples(1, s);
@@ -695,7 +698,7 @@ double optimize_layout_small(float* emb, int64_t n_vertices, int dim, const Grap
     p.next_neg = dneg.get();
     p.color_ptr = dptr.get();
     p.n_colors = n_colors;
-    p.events = reinterpret_cast<Event*>(work.get());
+    p.events = static_cast<Event*>(work.ptr);
     p.n_neg = reinterpret_cast<uint32_t*>(p.events + block * m);
     p.start = p.n_neg + block * m;
     p.rank_h = p.start + block * m;
@@ -758,6 +761,7 @@ double optimize_layout_small(float* emb, int64_t n_vertices, int dim, const Grap
     UMAPB_CUDA(cudaMemcpyAsync(&count, samples.get(), 8, cudaMemcpyDeviceToHost, s));
     UMAPB_CUDA(cudaMemcpyAsync(&failed, err.get(), 4, cudaMemcpyDeviceToHost, s));
     UMAPB_CUDA(cudaStreamSynchronize(s));
+    work.keep(kBlockBytes);
     if (failed) throw Error(UMAPB_ERR_CUDA, "the small-graph layout stopped on a wait limit");
     return static_cast<double>(count);
 }
