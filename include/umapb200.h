@@ -169,6 +169,10 @@ int32_t umapb_should_use_approximate_knn(const umapb_params* params, int64_t n_r
 /* ---- model lifecycle: UmapCore.__new__ (umap_rs/src/lib.rs:549-630) ---- */
 
 int32_t umapb_create(const umapb_params* params, umapb_model** out_model);
+/* Frees the model.  A call that leaves no model alive also gives back what the
+ * process keeps between calls: one block of work space (at most 256 MB of
+ * device memory) and one set of pinned upload buffers (8 MB).  `model` may be
+ * NULL, for a process that has used only the calls without a model. */
 void umapb_destroy(umapb_model* model);
 
 /* ---- fit / transform --------------------------------------------------- */

@@ -79,3 +79,10 @@ def test_ann_switch_matches_reference_pins(pins):
     p.use_approximate_knn = 1
     p.approx_knn_threshold = 0
     assert lib.umapb_should_use_approximate_knn(ctypes.byref(p), 2, 64) == 1
+
+
+def test_destroying_no_model_is_allowed():
+    lib = _lib.load()
+    lib.umapb_destroy(None)
+    test_create_destroy_needs_no_device()
+    lib.umapb_destroy(None)

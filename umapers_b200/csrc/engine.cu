@@ -1059,8 +1059,7 @@ void destroy_model(umapb_model* m) {
 }  // namespace
 
 void umapb_destroy(umapb_model* m) {
-    if (!m) return;
-    destroy_model(m);
+    if (m) destroy_model(m);
     if (g_models.load() == 0) trim_host_staging();
 }
 

@@ -23,7 +23,8 @@ constexpr size_t kStageBuf = static_cast<size_t>(1) << 20;
 constexpr int kStageThreads = 4;
 constexpr int kStageBufs = 2;
 // Pinned sets in use at once; a further upload takes the driver's copy.  One
-// is kept when idle, until the last model is destroyed.
+// (8 MB) is kept when idle, also by calls that make no model, until
+// umapb_destroy next leaves no model alive.
 constexpr int kStageSets = 2;
 
 struct StageSet {
