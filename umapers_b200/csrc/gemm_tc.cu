@@ -46,8 +46,8 @@ constexpr int kStages = 3;
 // and 5.16.  Below about 300,000 rows of 512 columns that wait costs more than
 // the overlap gains (150,000 rows beside a transform: 1.67 ms with two tiles,
 // 1.63 with one), and with one tile the second group is left out.
-constexpr int64_t kTilesPerStep = 4736;  // 32 per SM
-constexpr int64_t kMaxTilesPerCta = 4;
+constexpr uint32_t kTilesPerStep = 4736;  // 32 per SM
+constexpr uint32_t kMaxTilesPerCta = 4;
 constexpr int kTileBytes = GM * kBK * 2;         // 16 KiB per operand k-block
 constexpr int kStageBytes = 2 * kTileBytes;      // A + B
 constexpr uint32_t kGemmIdesc = idesc_bf16(GM, GN);
@@ -55,9 +55,9 @@ constexpr uint32_t kGemmIdesc = idesc_bf16(GM, GN);
 struct GemmParams {
     int64_t M, N;
     int kb;           // K / 64
-    int64_t n_tiles;  // column tiles
-    int64_t tiles;
-    int per_cta;      // tiles of a CTA
+    uint32_t n_tiles;  // column tiles
+    uint32_t tiles;    // below 2^31
+    uint32_t per_cta;  // tiles of a CTA
     GemmOut o;
 };
 
@@ -90,7 +90,7 @@ __device__ __forceinline__ void store_f32x32(float* dst, const float* v) {
     for (int q = 0; q < 8; ++q) d4[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
 }
 
-template <int EPI>
+template <int EPI, bool kFree>
 __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, int64_t row,
                                          int64_t n0, int64_t tile_n, uint32_t b_free) {
     const bool rv = row < p.M;
@@ -105,7 +105,7 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, in
         uint32_t r[32];
         tmem_ld32(taddr + 32 * c, r);
         tmem_wait_ld();
-        if (c == GN / 32 - 1) {  // the accumulator is read: the next tile may have it
+        if (kFree && c == GN / 32 - 1) {  // the accumulator is read: the next tile may have it
             fence_before();
             __syncwarp();
             if ((threadIdx.x & 31) == 0) mbar_arrive(b_free);
@@ -196,8 +196,9 @@ __device__ __forceinline__ void epilogue(const GemmParams& p, uint32_t taddr, in
 }
 
 template <int EPI, int kGroups>
-// registers: two CTAs an SM of 192 threads or of 320
-__global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
+// two CTAs an SM; with one group they fit without asking, and asking makes
+// kEpiGeluBwd spill
+__global__ void __launch_bounds__(64 + 128 * kGroups, kGroups)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 GemmParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -231,8 +232,9 @@ __global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
     __syncthreads();
     fence_after();
     const uint32_t tmem_base = *tmem_holder;
-    const int64_t first = static_cast<int64_t>(blockIdx.x) * p.per_cta;
-    const int64_t end = min(first + p.per_cta, p.tiles);
+    // with one group a CTA has one tile
+    const uint32_t first = kGroups == 1 ? blockIdx.x : blockIdx.x * p.per_cta;
+    const uint32_t end = kGroups == 1 ? first + 1 : min(first + p.per_cta, p.tiles);
 
     auto fail = [&](int code) {
         *abort_flag = 1;
@@ -243,7 +245,7 @@ __global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
         if (lane == 0) {
             uint32_t step = 0;  // k-blocks so far
             bool ok = true;
-            for (int64_t tile = first; ok && tile < end; ++tile) {
+            for (uint32_t tile = first; ok && tile < end; ++tile) {
                 const int m0 = static_cast<int>(tile / p.n_tiles) * GM;
                 const int n0 = static_cast<int>(tile % p.n_tiles) * GN;
                 for (int kb = 0; kb < p.kb; ++kb, ++step) {
@@ -264,9 +266,9 @@ __global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
         if (lane == 0) {
             uint32_t step = 0, seq = 0;
             bool ok = true;
-            for (int64_t tile = first; ok && tile < end; ++tile, ++seq) {
+            for (uint32_t tile = first; ok && tile < end; ++tile, ++seq) {
                 const uint32_t buf = seq % kGroups;
-                if (!mbar_wait(b_tempty + 8 * buf, ((seq / kGroups) & 1) ^ 1, abort_flag)) {
+                if (kGroups > 1 && !mbar_wait(b_tempty + 8 * buf, ((seq / kGroups) & 1) ^ 1, abort_flag)) {
                     fail(4);
                     break;
                 }
@@ -293,16 +295,17 @@ __global__ void __maxnreg__(kGroups == 1 ? 168 : 96)
     } else {
         const int quarter = warp & 3, group = (warp - 2) >> 2;
         uint32_t round = 0;
-        for (int64_t tile = first + group; tile < end; tile += kGroups, ++round) {
+        for (uint32_t tile = first + group; tile < end; tile += kGroups, ++round) {
+            const uint32_t tile_m = tile / p.n_tiles, tile_n = tile - tile_m * p.n_tiles;
             if (!mbar_wait(b_tfull + 8 * group, round & 1, abort_flag)) {
                 if (lane == 0) fail(3);
                 break;
             }
             fence_after();
-            const int64_t tile_n = tile % p.n_tiles;
-            epilogue<EPI>(p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * GN,
-                          (tile / p.n_tiles) * GM + quarter * 32 + lane, tile_n * GN, tile_n,
-                          b_tempty + 8 * group);
+            epilogue<EPI, (kGroups > 1)>(
+                p, tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + group * GN,
+                static_cast<int64_t>(tile_m) * GM + quarter * 32 + lane,
+                static_cast<int64_t>(tile_n) * GN, tile_n, b_tempty + 8 * group);
         }
     }
 
@@ -332,9 +335,18 @@ void launch_groups(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParam
     UMAPB_LAUNCH_CHECK();
 }
 
+// The two epilogues that only training uses keep one tile a CTA: at the 96
+// registers of two groups they spill.
 template <int EPI>
-void launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t s) {
-    p.per_cta == 1 ? launch_groups<EPI, 1>(ma, mb, p, s) : launch_groups<EPI, 2>(ma, mb, p, s);
+void launch(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams& p, cudaStream_t s) {
+    if constexpr (EPI != kEpiF32 && EPI != kEpiGeluBwd) {
+        p.per_cta = std::max(1u, std::min(kMaxTilesPerCta, p.tiles / kTilesPerStep));
+        if (p.per_cta > 1) {
+            launch_groups<EPI, 2>(ma, mb, p, s);
+            return;
+        }
+    }
+    launch_groups<EPI, 1>(ma, mb, p, s);
 }
 
 }  // namespace
@@ -352,13 +364,13 @@ void gemm_bf16_tn(const __nv_bfloat16* A, const __nv_bfloat16* B, int64_t M, int
     p.M = M;
     p.N = N;
     p.kb = static_cast<int>(K / kBK);
-    p.n_tiles = ceil_div(N, static_cast<int64_t>(GN));
     p.o = out;
     if (epilogue == kEpiRowMin && p.o.n_valid == 0) p.o.n_valid = N;
-    const int64_t m_tiles = ceil_div(M, static_cast<int64_t>(GM));
-    p.tiles = m_tiles * p.n_tiles;
-    p.per_cta = static_cast<int>(std::max<int64_t>(1, std::min(kMaxTilesPerCta, p.tiles / kTilesPerStep)));
-    if (p.tiles > 0x7FFFFFFFll) invalid("gemm_bf16_tn: too many tiles");
+    const int64_t n_tiles = ceil_div(N, GN), tiles = ceil_div(M, GM) * n_tiles;
+    if (tiles > 0x7FFFFFFFll) invalid("gemm_bf16_tn: too many tiles");
+    p.n_tiles = static_cast<uint32_t>(n_tiles);
+    p.tiles = static_cast<uint32_t>(tiles);
+    p.per_cta = 1;
     const CUtensorMap ma = make_bf16_map(A, M, K, GM);
     const CUtensorMap mb = make_bf16_map(B, N, K, GN);
     switch (epilogue) {

@@ -123,7 +123,7 @@ void knn_sparse(const CsrDevice& q, const CsrDevice& r, const CsrIndex& ri, bool
 // ------------------------------------------------------------ gemm_tc.cu
 // C[M x N] = A[M x K] B[N x K]^T on tcgen05 tensor cores: BF16 operands
 // (row-major, K contiguous, K % 64 == 0, 16-byte aligned), FP32 accumulation
-// in TMEM, one 128 x 128 output tile per CTA, and a fused epilogue.
+// in TMEM, one to four 128 x 128 output tiles per CTA, and a fused epilogue.
 enum GemmEpilogue : int {
     kEpiF32 = 0,           // c = A B^T                                 (fp32, ld N)
     kEpiBiasGelu = 1,      // z = A B^T + bias (fp32, optional); act = bf16(gelu(z)); act_t
