@@ -139,3 +139,23 @@ def test_a_null_array_is_an_error(n):
     assert lib.umapb_knn_query(None, n, gu._p(r), 50, 16, k, 0, 0, gu._p(idx), gu._p(dist)) != 0
     assert lib.umapb_knn_query(gu._p(r), 50, None, n, 16, k, 0, 0, gu._p(idx), gu._p(dist)) != 0
     _self_neighbours(r, np.arange(50))
+
+
+# indices up to the 16,384 that the host widens, and one query more
+@pytest.mark.parametrize("nq", [1, 512, 513])
+def test_few_indices_are_widened_on_the_host(nq):
+    test_indices_are_widened_chunk_by_chunk(nq + 1)
+    rng = np.random.default_rng(nq)
+    r = rng.standard_normal((500, 8), np.float32)
+    q = rng.standard_normal((nq, 8), np.float32)
+    idx, dist = gu.knn_query(q, r, 32)
+    full = np.sqrt(((q[:, None, :].astype(np.float64) - r[None]) ** 2).sum(-1))
+    # each row's distances, looked up by the indices, are the ones returned
+    assert np.abs(np.take_along_axis(full, idx, 1) - dist).max() <= 1e-5
+    assert np.abs(np.sort(full, 1)[:, :32] - dist).max() <= 1e-5
+
+
+# as many nonzeros as the host narrows, and one row more
+@pytest.mark.parametrize("n_rows", [32, 33])
+def test_few_column_indices_are_narrowed_on_the_host(n_rows):
+    test_column_indices_are_narrowed_chunk_by_chunk(n_rows)

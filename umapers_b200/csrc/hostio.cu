@@ -151,8 +151,11 @@ cudaError_t upload_staged(StageSet& set, char* dst, const char* src, size_t byte
 // Widened or narrowed on the device, kIndexChunk at a time, so the host makes
 // no pass over them and the scratch is 16 MB whatever the count.  With 1.8M
 // indices out (60,013 rows, k = 30) the call takes 7.3 ms; through a host
-// vector of 32-bit indices it took 9.1.
+// vector of 32-bit indices it took 9.1.  Up to kHostIndices the host vector is
+// kept: a buffer and a launch are 10 us of a call of 250 (500 rows, one query),
+// and from 10,000 to 65,000 indices the two are level.
 constexpr int64_t kIndexChunk = 2 << 20;
+constexpr int64_t kHostIndices = 1 << 14;
 
 template <typename From, typename To>
 __global__ void convert_kernel(const From* __restrict__ in, int64_t n, To* __restrict__ out) {
@@ -194,6 +197,12 @@ void trim_host_staging() {
 }
 
 void download_indices(int64_t* dst, const int32_t* src, int64_t n, cudaStream_t s) {
+    if (n <= kHostIndices) {
+        std::vector<int32_t> narrow(n);  // pageable: the copy has been made when the call returns
+        UMAPB_CUDA(cudaMemcpyAsync(narrow.data(), src, n * 4, cudaMemcpyDeviceToHost, s));
+        std::copy(narrow.begin(), narrow.end(), dst);
+        return;
+    }
     DevBuf<int64_t> wide(std::min(n, kIndexChunk), s);
     for (int64_t at = 0; at < n; at += kIndexChunk) {
         const int64_t len = std::min(kIndexChunk, n - at);
@@ -205,6 +214,12 @@ void download_indices(int64_t* dst, const int32_t* src, int64_t n, cudaStream_t 
 }
 
 void upload_indices(int32_t* dst, const int64_t* src, int64_t n, cudaStream_t s) {
+    if (n <= kHostIndices) {
+        std::vector<int32_t> narrow(src, src + n);
+        if (n > 0)
+            UMAPB_CUDA(cudaMemcpyAsync(dst, narrow.data(), n * 4, cudaMemcpyHostToDevice, s));
+        return;
+    }
     DevBuf<int64_t> wide(std::min(n, kIndexChunk), s);
     for (int64_t at = 0; at < n; at += kIndexChunk) {
         const int64_t len = std::min(kIndexChunk, n - at);
