@@ -114,3 +114,10 @@ def test_nndescent_follows_the_rule_step_by_step(orc, n, d, k, candidates, iters
     ref = replay(full, k, candidates, iters, 99)
     assert np.array_equal(gi, [[j for _, j in r] for r in ref])
     assert np.array_equal(gd, np.array([[v for v, _ in r] for r in ref], np.float32))
+
+
+# row lengths and list widths (256, 512 and 1,024 candidates) on both sides of
+# where whole 16-byte quads stop being read two lanes a candidate
+@pytest.mark.parametrize("d,k", [(800, 15), (804, 15), (480, 20), (484, 20), (804, 31)])
+def test_long_rows_follow_the_rule_step_by_step(orc, d, k):
+    test_nndescent_follows_the_rule_step_by_step(orc, 300, d, k, k, 2)

@@ -431,8 +431,8 @@ __device__ __forceinline__ uint64_t merge_best(uint64_t best, uint64_t chunk) {
     return x;
 }
 
-// The distances for rows that are not whole 16-byte quads: eval_candidates
-// on index and distance arrays.
+// eval_candidates on index and distance arrays, for rows that are not whole
+// 16-byte quads and for those too long for eval_quads (quads_pay).
 __device__ inline void eval_scalar(const float* __restrict__ X, const float* __restrict__ norms,
                                    int64_t i, int d, bool cosine, const float* qs,
                                    const uint32_t* cand, float* dist, int m) {
@@ -531,6 +531,19 @@ __device__ inline void eval_quads(const float* __restrict__ X, const float* __re
             dist[c] = dense_distance(sum, norms, i, j, cosine);
         }
     }
+}
+
+// Whether eval_quads is the faster form.  A warp of it reads 16 rows at a time and
+// eval_scalar 4, and what waits for L2 needs lines of the L1 cache, which is what
+// the query rows and candidates of the resident warps leave of 256 KB: 28 KB once
+// they take more than 196.  Long rows and wide lists therefore take eval_scalar;
+// at 1,024 candidates so few warps are resident that the wider form pays at any
+// length.  A run's iterations, ms, eval_quads / eval_scalar (30,000 rows):
+// k = 15 d = 800 16.3 / 17.0, 900 20.6 / 17.7, 1,000 35.9 / 19.6; k = 10 d = 800
+// 8.2 / 9.1, 1,000 12.2 / 11.0, 1,500 36.8 / 19.0; k = 20 d = 400 9.5 / 9.7, 500
+// 20.7 / 12.3, 800 33.7 / 22.5; k = 30 d = 500 15.6 / 18.7, 1,500 59.0 / 69.9.
+inline bool quads_pay(int cap, int d) {
+    return cap >= 1024 || d <= (cap == 512 ? 480 : 800);
 }
 
 template <bool SP>
@@ -819,7 +832,7 @@ int64_t nndescent(const float* X, int64_t n, int d, int k, int metric, int64_t c
     p.k = k;
     p.cosine = metric == UMAPB_METRIC_COSINE;
     p.metric = metric;
-    p.quads = d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    p.quads = quads_pay(p.cap, d) && d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     p.seed = seed;
     return nndescent_run<false>(p, n, k, n_iters, smem, out_idx, out_dist, s, stats);
 }
