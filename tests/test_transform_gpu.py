@@ -91,3 +91,14 @@ def test_transform_device_writes_to_any_float_address(n):
         _lib.check(_lib.load().umapb_transform_device(m._core._handle, qd.data_ptr(), n, 16, out))
     assert torch.equal(flat[1:-2].reshape(n, 2), want)
     assert flat[0] == -7.0 and (flat[-2:] == -7.0).all()
+
+
+def test_transform_at_the_largest_request_of_several_lanes():
+    # 14,208 queries fit the GPU at four lanes each, one more takes a thread
+    # each; whole copies of a request leave its largest weight and mean distance
+    fit, q = workloads.transform_mixture(n_fit=1500, n_query=7104, d=24, n_comp=6)
+    m = Umap(n_neighbors=15, n_epochs=20, random_seed=5)
+    m.fit(fit)
+    for n, few, many in ((7104, 2, 3), (1093, 12, 13)):  # 14,208; 14,209 = 13 x 1,093
+        a, b = (m.transform(np.tile(q[:n], (c, 1)))[:n] for c in (few, many))
+        assert np.array_equal(a, b)

@@ -838,7 +838,9 @@ __global__ void __launch_bounds__(kTransformThreads) transform_kernel(TransformA
 // edges in registers and, while the group works through one epoch's samples,
 // copies the next epoch's negatives into shared memory.  What is left on the
 // chain is the update itself (about 230 cycles a sample).
-constexpr int64_t kLanes16Queries = 4096, kLanes8Queries = 8192, kLanes4Queries = 16384;
+// The last limit is what fits the GPU at once: three CTAs of 32 queries (76 KB) an
+// SM.
+constexpr int64_t kLanes16Queries = 4096, kLanes8Queries = 8192, kLanes4Queries = 3 * 148 * 32;
 
 struct GroupStage {
     float2 tail[kStageEdges];
@@ -1612,8 +1614,11 @@ void transform_layout(float* out, int64_t nq, int dim, const float* base, int64_
     // schedulers keep a few warps each.  100 epochs on a 4,000-row fit, ms at
     // 1 / 3,000 / 6,000 / 10,000 queries: one thread 1.75 / 2.64 / 2.54 / 2.55, 4
     // lanes 1.29 / 1.80 / 1.88 / 2.13, 8 lanes 1.18 / 1.65 / 1.79 / 2.49, 16 lanes
-    // 1.11 / 1.54 / 2.51 / 3.56; 30 epochs at 35,000 queries: one thread 0.72,
-    // 4 lanes 1.48.
+    // 1.11 / 1.54 / 2.51 / 3.56; at 14,000 one thread 3.24, 4 lanes 2.85 (whole
+    // calls), at 16,384, a second round of CTAs, 3.31 and 4.46.  Queries of more
+    // than kStageEdges edges (k = 20 and 30 there, whole calls, one thread / lanes):
+    // 100 queries 8.8 / 5.2 and 12.5 / 7.0, 3,000 8.4 / 6.0 and 12.1 / 8.1, 6,000
+    // 8.3 / 8.3 and 12.1 / 11.6, level at 12,000.
     if (dim == 2 && nq <= kLanes16Queries)
         group(transform_group_kernel<16>, 16, sizeof(GroupStage));
     else if (dim == 2 && nq <= kLanes8Queries)
