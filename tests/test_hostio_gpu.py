@@ -159,3 +159,36 @@ def test_few_indices_are_widened_on_the_host(nq):
 @pytest.mark.parametrize("n_rows", [32, 33])
 def test_few_column_indices_are_narrowed_on_the_host(n_rows):
     test_column_indices_are_narrowed_chunk_by_chunk(n_rows)
+
+
+# an odd number of indices goes through the distances' memory in three pieces,
+# and distances come out before their memory is used
+@pytest.mark.parametrize("nq,k", [(16_385, 1), (5_463, 3), (99_999, 5)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_indices_are_widened_through_the_memory_of_the_distances(nq, k, pinned):
+    rng = np.random.default_rng(nq)
+    r, q = rng.standard_normal((300, 5), np.float32), rng.standard_normal((nq, 5), np.float32)
+    idx = torch.full((nq, k), -1, dtype=torch.int64)
+    dist = torch.full((nq, k), -1.0)
+    if pinned:
+        idx, dist = idx.pin_memory(), dist.pin_memory()
+    idx, dist = idx.numpy(), dist.numpy()
+    _lib.check(_lib.load().umapb_knn_query(gu._p(q), nq, gu._p(r), 300, 5, k, 0, 0, gu._p(idx),
+                                           gu._p(dist)))
+    full = np.sqrt(((q[:, None, :].astype(np.float64) - r[None]) ** 2).sum(-1))
+    assert np.abs(np.take_along_axis(full, idx, 1) - dist).max() <= 1e-5
+    assert np.abs(np.sort(full, 1)[:, :k] - dist).max() <= 1e-5
+
+
+def test_an_odd_number_of_column_indices_is_narrowed():
+    per_row, n_rows, n_cols, k = 5, 3277, 40, 3  # 16,385 nonzeros
+    ip, ix, dv = _csr(n_rows, per_row, n_cols, 3)
+    dense = np.zeros((n_rows, n_cols), np.float32)
+    dense[np.repeat(np.arange(n_rows), per_row), ix] = dv
+    idx, dist = np.empty((n_rows, k), np.int64), np.empty((n_rows, k), np.float32)
+    _lib.check(_lib.load().umapb_knn_csr(gu._p(ip), gu._p(ix), gu._p(dv), n_rows, n_cols, k, 0,
+                                         gu._p(idx), gu._p(dist)))
+    want = gu.knn_exact(dense, k)[1]
+    # squared distances up to 40 as sums in two orders, 10 products each: 40 * 20 * 6e-8
+    # apart, and the root of a difference as small as that
+    assert np.abs(dist - want).max() <= np.sqrt(40 * 20 * 6e-8)

@@ -1435,8 +1435,7 @@ int32_t umapb_knn_exact(const float* data, int64_t n, int64_t d, int64_t k, int3
         int64_t fb = 0;
         knn_exact_device(X.get(), n, X.get(), n, static_cast<int>(d), static_cast<int>(k), metric,
                          backend, idx.get(), dist.get(), &fb, nullptr, nullptr, ss.s);
-        download_indices(indices, idx.get(), n * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_neighbors(indices, dists, idx.get(), dist.get(), n * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
         if (fallback_rows) *fallback_rows = fb;
     });
@@ -1457,8 +1456,7 @@ int32_t umapb_knn_query(const float* query, int64_t nq, const float* reference, 
         DevBuf<float> dist(nq * k, ss.s);
         knn_exact_device(Q.get(), nq, R.get(), nr, static_cast<int>(d), static_cast<int>(k),
                          metric, backend, idx.get(), dist.get(), nullptr, nullptr, nullptr, ss.s);
-        download_indices(indices, idx.get(), nq * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), nq * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_neighbors(indices, dists, idx.get(), dist.get(), nq * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
     });
 }
@@ -1478,9 +1476,7 @@ int32_t umapb_knn_csr(const int64_t* indptr, const int64_t* indices, const float
         DevBuf<int32_t> idx(n_rows * k, ss.s);
         DevBuf<float> dist(n_rows * k, ss.s);
         knn_sparse(csr, csr, ci, true, static_cast<int>(k), metric, idx.get(), dist.get(), ss.s);
-        download_indices(out_idx, idx.get(), n_rows * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_neighbors(out_idx, out_dist, idx.get(), dist.get(), n_rows * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
     });
 }
@@ -1502,9 +1498,7 @@ int32_t umapb_nndescent_csr(const int64_t* indptr, const int64_t* indices, const
         NdStats st;
         const int64_t ran = nndescent_csr(csr, static_cast<int>(k), metric, candidate_pool,
                                           n_iters, seed, idx.get(), dist.get(), ss.s, &st);
-        download_indices(out_idx, idx.get(), n_rows * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_rows * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_neighbors(out_idx, out_dist, idx.get(), dist.get(), n_rows * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
         if (iters_run) *iters_run = ran;
         if (candidates_evaluated) *candidates_evaluated = st.candidates;
@@ -1531,9 +1525,7 @@ int32_t umapb_knn_csr_query(const int64_t* q_indptr, const int64_t* q_indices,
         DevBuf<int32_t> idx(n_q * k, ss.s);
         DevBuf<float> dist(n_q * k, ss.s);
         knn_sparse(q, r, ri, false, static_cast<int>(k), metric, idx.get(), dist.get(), ss.s);
-        download_indices(out_idx, idx.get(), n_q * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(out_dist, dist.get(), n_q * k * 4, cudaMemcpyDeviceToHost,
-                                   ss.s));
+        download_neighbors(out_idx, out_dist, idx.get(), dist.get(), n_q * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
     });
 }
@@ -1557,8 +1549,7 @@ int32_t umapb_nndescent(const float* data, int64_t n, int64_t d, int64_t k, int3
                                              dist.get(), ss.s, &st);
         if (candidates_evaluated) *candidates_evaluated = st.candidates;
         if (kernel_sec) *kernel_sec = st.kernel_sec;
-        download_indices(indices, idx.get(), n * k, ss.s);
-        UMAPB_CUDA(cudaMemcpyAsync(dists, dist.get(), n * k * 4, cudaMemcpyDeviceToHost, ss.s));
+        download_neighbors(indices, dists, idx.get(), dist.get(), n * k, ss.s);
         UMAPB_CUDA(cudaStreamSynchronize(ss.s));
         if (iters_run) *iters_run = ran;
     });

@@ -148,13 +148,11 @@ cudaError_t upload_staged(StageSet& set, char* dst, const char* src, size_t byte
 }
 
 // ------------------------------------------------------- 64-bit indices
-// Widened or narrowed on the device, kIndexChunk at a time, so the host makes
-// no pass over them and the scratch is 16 MB whatever the count.  With 1.8M
-// indices out (60,013 rows, k = 30) the call takes 7.3 ms; through a host
-// vector of 32-bit indices it took 9.1.  Up to kHostIndices the host vector is
-// kept: a buffer and a launch are 10 us of a call of 250 (500 rows, one query),
-// and from 10,000 to 65,000 indices the two are level.
-constexpr int64_t kIndexChunk = 2 << 20;
+// Widened or narrowed on the device, through the memory of the floats that go
+// with them (one a index), so the host makes no pass over them and nothing is
+// allocated.  With 1.8M indices out (60,013 rows, k = 30) the call takes 7.3 ms;
+// through a host vector of 32-bit indices it took 9.1.  Up to kHostIndices the
+// host vector is kept: two more copies and launches are as long.
 constexpr int64_t kHostIndices = 1 << 14;
 
 template <typename From, typename To>
@@ -196,38 +194,41 @@ void trim_host_staging() {
     delete set;
 }
 
-void download_indices(int64_t* dst, const int32_t* src, int64_t n, cudaStream_t s) {
+void download_neighbors(int64_t* idx_out, float* dist_out, const int32_t* idx, float* dist,
+                        int64_t n, cudaStream_t s) {
+    if (!idx_out) throw_cuda(cudaErrorInvalidValue, "download to a null host array", __FILE__, __LINE__);
+    UMAPB_CUDA(cudaMemcpyAsync(dist_out, dist, n * 4, cudaMemcpyDeviceToHost, s));
     if (n <= kHostIndices) {
         std::vector<int32_t> narrow(n);  // pageable: the copy has been made when the call returns
-        UMAPB_CUDA(cudaMemcpyAsync(narrow.data(), src, n * 4, cudaMemcpyDeviceToHost, s));
-        std::copy(narrow.begin(), narrow.end(), dst);
+        UMAPB_CUDA(cudaMemcpyAsync(narrow.data(), idx, n * 4, cudaMemcpyDeviceToHost, s));
+        std::copy(narrow.begin(), narrow.end(), idx_out);
         return;
     }
-    DevBuf<int64_t> wide(std::min(n, kIndexChunk), s);
-    for (int64_t at = 0; at < n; at += kIndexChunk) {
-        const int64_t len = std::min(kIndexChunk, n - at);
-        convert_kernel<<<static_cast<unsigned>(ceil_div(len, 256)), 256, 0, s>>>(src + at, len,
-                                                                                 wide.get());
+    int64_t* wide = reinterpret_cast<int64_t*>(dist);
+    for (int64_t at = 0, len = n / 2; at < n; at += len) {
+        len = std::min(len, n - at);
+        convert_kernel<<<static_cast<unsigned>(ceil_div(len, 256)), 256, 0, s>>>(idx + at, len, wide);
         UMAPB_LAUNCH_CHECK();
-        UMAPB_CUDA(cudaMemcpyAsync(dst + at, wide.get(), len * 8, cudaMemcpyDeviceToHost, s));
+        UMAPB_CUDA(cudaMemcpyAsync(idx_out + at, wide, len * 8, cudaMemcpyDeviceToHost, s));
     }
 }
 
-void upload_indices(int32_t* dst, const int64_t* src, int64_t n, cudaStream_t s) {
+void upload_columns(int32_t* idx, float* values, const int64_t* idx_in, const float* values_in,
+                    int64_t n, cudaStream_t s) {
     if (n <= kHostIndices) {
-        std::vector<int32_t> narrow(src, src + n);
+        std::vector<int32_t> narrow(idx_in, idx_in + n);
         if (n > 0)
-            UMAPB_CUDA(cudaMemcpyAsync(dst, narrow.data(), n * 4, cudaMemcpyHostToDevice, s));
-        return;
+            UMAPB_CUDA(cudaMemcpyAsync(idx, narrow.data(), n * 4, cudaMemcpyHostToDevice, s));
+    } else {
+        int64_t* wide = reinterpret_cast<int64_t*>(values);
+        for (int64_t at = 0, len = n / 2; at < n; at += len) {
+            len = std::min(len, n - at);
+            upload_host(wide, idx_in + at, len * 8, s);
+            convert_kernel<<<static_cast<unsigned>(ceil_div(len, 256)), 256, 0, s>>>(wide, len, idx + at);
+            UMAPB_LAUNCH_CHECK();
+        }
     }
-    DevBuf<int64_t> wide(std::min(n, kIndexChunk), s);
-    for (int64_t at = 0; at < n; at += kIndexChunk) {
-        const int64_t len = std::min(kIndexChunk, n - at);
-        UMAPB_CUDA(cudaMemcpyAsync(wide.get(), src + at, len * 8, cudaMemcpyHostToDevice, s));
-        convert_kernel<<<static_cast<unsigned>(ceil_div(len, 256)), 256, 0, s>>>(wide.get(), len,
-                                                                                 dst + at);
-        UMAPB_LAUNCH_CHECK();
-    }
+    upload_host(values, values_in, n * 4, s);
 }
 
 }  // namespace umapb

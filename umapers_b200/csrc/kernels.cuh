@@ -76,8 +76,12 @@ struct CsrDevice {
 // rules: pinned arrays are in use until `s` has been synchronised.
 int host_threads();
 void upload_host(void* dst, const void* src, size_t bytes, cudaStream_t s);
-void download_indices(int64_t* dst, const int32_t* src, int64_t n, cudaStream_t s);
-void upload_indices(int32_t* dst, const int64_t* src, int64_t n, cudaStream_t s);
+// n neighbour indices and their distances out, the indices widened; `dist` (device)
+// is overwritten.  n column indices and their values in, the indices narrowed.
+void download_neighbors(int64_t* idx_out, float* dist_out, const int32_t* idx, float* dist,
+                        int64_t n, cudaStream_t s);
+void upload_columns(int32_t* idx, float* values, const int64_t* idx_in, const float* values_in,
+                    int64_t n, cudaStream_t s);
 // Frees the pinned buffers that no upload is using.
 void trim_host_staging();
 

@@ -461,8 +461,7 @@ void csr_upload(const int64_t* indptr, const int64_t* indices, const float* valu
     upload_host(out.indptr.get(), indptr, (n_rows + 1) * 8, s);
     out.indices.alloc(std::max<int64_t>(nnz, 1), s);
     out.values.alloc(std::max<int64_t>(nnz, 1), s);
-    upload_indices(out.indices.get(), indices, nnz, s);
-    upload_host(out.values.get(), values, nnz * 4, s);
+    upload_columns(out.indices.get(), out.values.get(), indices, values, nnz, s);
     out.sq.alloc(std::max<int64_t>(n_rows, 1), s);
     out.l2.alloc(std::max<int64_t>(n_rows, 1), s);
     if (n_rows > 0) {
