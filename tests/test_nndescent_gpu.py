@@ -1,10 +1,12 @@
 """NN-descent on the GPU: recall against exact kNN (the reference's
 thresholds, rust_umap/src/lib.rs:6733-6764) and against the oracle's own
 recall on the same data."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from umapers_b200 import workloads
+from umapers_b200 import _lib, workloads
 from tests import gpu_util as gu
 
 pytestmark = pytest.mark.gpu
@@ -121,3 +123,58 @@ def test_nndescent_follows_the_rule_step_by_step(orc, n, d, k, candidates, iters
 @pytest.mark.parametrize("d,k", [(800, 15), (804, 15), (480, 20), (484, 20), (804, 31)])
 def test_long_rows_follow_the_rule_step_by_step(orc, d, k):
     test_nndescent_follows_the_rule_step_by_step(orc, 300, d, k, k, 2)
+
+
+def _against_the_rule(got, full, k, candidates, iters, seed):
+    gi, gd = got
+    ref = replay(full, k, candidates, iters, seed)
+    assert np.array_equal(gi, [[j for _, j in r] for r in ref])
+    assert np.array_equal(gd, np.array([[v for v, _ in r] for r in ref], np.float32))
+
+
+@pytest.mark.parametrize("n,d,k,candidates,iters", [
+    (40, 6, 2, 4, 3), (150, 63, 5, 5, 2), (200, 64, 10, 12, 2), (300, 60, 15, 15, 2),
+    (300, 101, 15, 50, 2), (260, 72, 22, 22, 2), (300, 66, 31, 40, 2), (300, 804, 15, 15, 2)])
+def test_cosine_rows_follow_the_rule_step_by_step(orc, n, d, k, candidates, iters):
+    # the forms of four rows and of sixteen, narrow and wide rows, with and
+    # without a tail; a zero row and a repeated one
+    x = np.random.default_rng(d).normal(size=(n, d)).astype(np.float32)
+    x[5], x[7] = 0.0, 2.0 * x[6]
+    idx, dist = orc.exact_knn(x, n, metric="cosine")
+    full = np.empty((n, n), np.float32)
+    np.put_along_axis(full, idx.astype(np.int64), dist, axis=1)
+    got = gu.nndescent(x, k, candidates, iters, 99, metric="cosine")[:2]
+    _against_the_rule(got, full, k, candidates, iters, 99)
+
+
+@pytest.mark.parametrize("metric", ["euclidean", "cosine"])
+@pytest.mark.parametrize("n,nnz,k,candidates", [(40, 3, 2, 4), (150, 4, 5, 5), (200, 13, 10, 12),
+                                                (300, 21, 15, 50), (260, 30, 22, 22),
+                                                (300, 7, 31, 31), (300, 33, 31, 40)])
+def test_csr_rows_follow_the_rule_step_by_step(n, nnz, k, candidates, metric):
+    # every register width on CSR rows; the longest row is and is not a
+    # multiple of four, some rows are empty
+    rng, d, iters, seed = np.random.default_rng(n + nnz), 3 * nnz, 2, 99
+    counts = rng.integers(0, nnz + 1, n)
+    counts[3], counts[11] = nnz, 0
+    ip = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    ix = np.concatenate([np.sort(rng.choice(d, c, replace=False)) for c in counts]).astype(np.int64)
+    dv = rng.lognormal(0.0, 1.0, len(ix)).astype(np.float32)
+    lib, m = _lib.load(), gu.METRIC[metric]
+    # all distances from the exact sparse kNN, 20 reference rows at a time
+    full = np.empty((n, n), np.float32)
+    for r0 in range(0, n, 20):
+        c = min(20, n - r0)
+        rp = ip[r0:r0 + c + 1] - ip[r0]
+        rx, rv = ix[ip[r0]:ip[r0 + c]], dv[ip[r0]:ip[r0 + c]]
+        i, v = np.empty((n, c), np.int64), np.empty((n, c), np.float32)
+        _lib.check(lib.umapb_knn_csr_query(gu._p(ip), gu._p(ix), gu._p(dv), n, gu._p(rp),
+                                           gu._p(rx), gu._p(rv), c, d, c, m, gu._p(i), gu._p(v)))
+        np.put_along_axis(full, r0 + i, v, axis=1)
+    np.fill_diagonal(full, 0.0)
+    gi, gd = np.empty((n, k), np.int64), np.empty((n, k), np.float32)
+    ran, ev, sec = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_double()
+    _lib.check(lib.umapb_nndescent_csr(gu._p(ip), gu._p(ix), gu._p(dv), n, d, k, m, candidates,
+                                       iters, seed, gu._p(gi), gu._p(gd), ctypes.byref(ran),
+                                       ctypes.byref(ev), ctypes.byref(sec)))
+    _against_the_rule((gi, gd), full, k, candidates, iters, seed)
