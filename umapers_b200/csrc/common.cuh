@@ -60,14 +60,12 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Lets a kernel be launched with any dynamic shared memory that fits a block.
 // A kernel's limit belongs to the process, so a call that set it to its own size
 // could lower it between another thread's setting and launch; this sets the
-// same value every time.
+// same value every time.  `statics`: at least what the kernel has besides.
 template <typename Kernel>
-void allow_shared(Kernel* kernel) {
+void allow_shared(Kernel* kernel, int statics = 0) {
     constexpr int kBlockShared = 227 * 1024;
-    cudaFuncAttributes fa{};
-    UMAPB_CUDA(cudaFuncGetAttributes(&fa, kernel));
     UMAPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kBlockShared - static_cast<int>(fa.sharedSizeBytes)));
+                                    kBlockShared - statics));
 }
 
 // Blocks released by DevBuf are kept per (device, stream, exact size) and

@@ -273,7 +273,7 @@ void launch_plain(const float* Q, const int32_t* q_rows, int64_t n_q, const floa
                   cudaStream_t s, bool allow_scratch) {
     const size_t smem = plain_smem<QT, CT>(d, k);
     auto kern = knn_plain_kernel<QT, CT, COS>;
-    allow_shared(kern);
+    allow_shared(kern, 1024);
     const int64_t blocks = ceil_div(n_q, QT);
     int dev = 0, sms = 0;
     UMAPB_CUDA(cudaGetDevice(&dev));

@@ -727,8 +727,8 @@ double optimize_layout_small(float* emb, int64_t n_vertices, int dim, const Grap
                   : dim == 3 ? layout_kernel<3>
                   : dim == 4 ? layout_kernel<4>
                              : layout_kernel<0>;
-    allow_shared(order_kernel);
-    allow_shared(layout);
+    allow_shared(order_kernel, 1024);
+    allow_shared(layout, 1024);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (kernel_ms) {
         UMAPB_CUDA(cudaEventCreate(&e0));
