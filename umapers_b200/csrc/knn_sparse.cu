@@ -31,9 +31,10 @@
 //    stops once no later row can enter the full list.
 // In the self join a row's distance to itself is 0, as in the reference.
 //
-// Bound by instruction issue and fetch (ncu at 30,000 x 2,000: a third of the
-// stalls wait for instructions, L2 at 6%).  100,000 x 2,000 cosine rows, k =
-// 30: 21.5 -> 17.4 ms with (row, value) pairs in one load, 32-bit offsets, far
+// Bound by instruction issue and latency on the 16 warps an SM that the
+// accumulators leave (ncu at 30,000 x 2,000: issue active 52% of cycles; of 7.7
+// cycles an instruction 2.7 wait for fixed latencies, 1.5 for shared memory, 1.1
+// for L2, which runs at 9%).  100,000 x 2,000 cosine rows, k = 30: 21.5 -> 17.4 ms with (row, value) pairs in one load, 32-bit offsets, far
 // rows turned away before the division, and no walk over untouched rows that
 // cannot enter.  Walking the whole accumulator instead of a list of touched
 // rows gave 15.9 there but 1.2 instead of 0.7 ms at 20,000 x 8,000; more

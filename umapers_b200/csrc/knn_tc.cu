@@ -284,7 +284,9 @@ __device__ __forceinline__ uint64_t held_key(uint64_t raw) {
 // words are sorted instead of 64-bit keys.  A list then keeps 32 keys such
 // that every key left out has an L of at least the largest kept one's with
 // those bits cleared; the threshold and the re-rank's bound are taken from
-// that (2^-16 of L, far inside the slack of the error bound).  The kernel on
+// that (2^-16 of L, far inside the slack of the error bound: of 1M x 64 rows
+// 3,979 go to the second pass, 3,977 with whole keys, of 60,013 x 100 with cosine
+// and k = 30 2,265 and 2,261).  The kernel on
 // 300,000 queries of 8,000 x 128 rows, whose short walks are mostly merges,
 // 6.9 -> 6.0 ms; 1M x 64 199.9 -> 194.7.  What is left there is the appends: with
 // 32 rows a warp, some row is pending in most tiles.

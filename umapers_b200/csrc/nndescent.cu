@@ -367,9 +367,10 @@ __global__ void __launch_bounds__(kWarps * 32) nd_iter_kernel(NdArgs p, uint64_t
 // its swaps one after another (a lane drew and swapped 201 times on its own);
 // distances load 16 bytes at a time; and the k best come from a 32-entry list
 // instead of a second sort.  Bound by the gathers of candidate rows:
-// 100,003 x 100 rows, k = 15, 50 candidates, 14 iterations (2.5e8 candidates of
-// 400 bytes) 38.6 -> 18.6 ms, 5.4 TB/s; 200,000 x 64, 10 iterations 42.8 -> 16.0;
-// 8,000 x 100, k = 30 7.6 -> 2.1; 20,000 CSR rows 5.2 -> 2.1.
+// 100,003 x 100 rows, k = 15, 50 candidates, 14 iterations (2.41e8 candidates of
+// 400 bytes) 18.1 ms, 5.3 TB/s, mostly from L2 (nd_iter_kernel 38.6); 200,000 x 64,
+// 10 iterations 16.0 (42.8); 8,000 x 100, k = 30 2.1 (7.6); 20,000 CSR rows 2.1
+// (5.2).
 
 // Ascending bitonic sort of 32 * NPL values, element NPL * lane + r in v[r].
 template <int NPL>

@@ -18,8 +18,8 @@
 //                  edge its rank among its head's and its tail's due edges and
 //                  the earliest time it could start, and writes one 48-byte
 //                  event per due edge, sorted by that time, in batches of up
-//                  to 32 that could start together (0.2 ms for 148 epochs of
-//                  1,000 rows, 0.5 ms for 100 epochs of 4,200 rows);
+//                  to 32 that could start together (0.24 ms a block of epochs
+//                  at 1,000 rows, 0.6 at 4,200);
 //   layout_kernel  one CTA holds the embedding in shared memory and runs the
 //                  batches of the block's epochs.  A warp takes a batch, waits
 //                  until each event's two vertices have reached its ranks,
@@ -28,19 +28,20 @@
 // What bounds it is the serial chain of the busiest vertex: about 390 cycles
 // for an attractive step and 270 for a negative (logarithm 64, exponential,
 // division 40 and a dozen dependent operations), behind about 200 cycles from
-// one warp's store to the next one's start.  At 1,000 x 32 (22,500 edges, 6,900
-// due in an epoch, a vertex with 39 due edges at its head and as many at its
-// tail) that is at least 60 us an epoch; it takes 137.  The form this replaced
-// put a barrier after every colour (256 there, 646 at 4,200 x 96), and each
-// colour waited for its schedule from global memory and drew its random
-// numbers on the chain: 200 epochs of 1,000 x 32 took 224 ms, now 27; 100
-// epochs of 4,200 x 96 took 278 ms, now 40; of 8,192 x 32 282 ms, now 39.
+// one warp's store to the next one's start.  At 1,000 x 32 rows of noise (22,500
+// edges, 6,900 due in an epoch; by the rows drawn, a vertex with 37 to 55 due
+// edges at its head and as many at its tail) the arithmetic of that chain is 41
+// to 61 us an epoch; layout_kernel takes 119 to 164.  The three kernels
+// together, against one CTA with a barrier after every colour that reads its
+// schedule and draws its random numbers on the chain: 200 epochs of 1,000 x 32
+// (55 due edges) 33.4 and 272 ms, 100 epochs of 4,200 x 96 34.9 and 282, of
+// 8,192 x 32 42.9 and 286.
 //
-// Measured and not kept (1,000 x 32 / 4,200 x 96, ms as above): the events in
-// colour order, one per lane (53 / 62); each ready lane at once instead of the
-// whole batch together (36 / 48); a state machine that runs one sample of
-// every lane's event a step (44 / 60: its polls, votes and branches cost more
-// than the step); smaller batches (38 / 50 at half the size).
+// Measured and not kept (1,000 x 32 / 4,200 x 96, against 27 / 40 ms on the same
+// rows): the events in colour order, one per lane (53 / 62); each ready lane at
+// once instead of the whole batch together (36 / 48); a state machine that runs
+// one sample of every lane's event a step (44 / 60: its polls, votes and branches
+// cost more than the step); smaller batches (38 / 50 at half the size).
 //
 // A wait always ends: batches are in an order that respects the dependencies
 // and a warp takes its own in that order, so the first batch that is not done
