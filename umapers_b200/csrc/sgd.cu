@@ -1615,7 +1615,7 @@ void transform_layout(float* out, int64_t nq, int dim, const float* base, int64_
     // 1 / 3,000 / 6,000 / 10,000 queries: one thread 1.75 / 2.64 / 2.54 / 2.55, 4
     // lanes 1.29 / 1.80 / 1.88 / 2.13, 8 lanes 1.18 / 1.65 / 1.79 / 2.49, 16 lanes
     // 1.11 / 1.54 / 2.51 / 3.56; at 14,000 one thread 3.24, 4 lanes 2.85 (whole
-    // calls), at 16,384, a second round of CTAs, 3.31 and 4.46.  Queries of more
+    // calls), at 16,384, a second wave of CTAs, 3.31 and 4.46.  Queries of more
     // than kStageEdges edges (k = 20 and 30 there, whole calls, one thread / lanes):
     // 100 queries 8.8 / 5.2 and 12.5 / 7.0, 3,000 8.4 / 6.0 and 12.1 / 8.1, 6,000
     // 8.3 / 8.3 and 12.1 / 11.6, level at 12,000.
